@@ -1,4 +1,4 @@
-// Register-resident forward DFT butterflies of radix 1, 2, 3, 4, 5, 7, 8, 16.
+// Register-resident forward DFT butterflies of radix 1 to 10, 12, 14, 15 and 16.
 //
 // All butterflies compute X_p = sum_q v_q * exp(-2*pi*i*p*q/R) in place on an array
 // of R complex values held in registers. Inverse transforms are obtained by the
@@ -57,6 +57,12 @@ template <class C> SFB_HD C cmake(decltype(C::x) x, decltype(C::x) y) { C r; r.x
 #define SFB_K7S1 0.781831482468029808708
 #define SFB_K7S2 0.974927912181823607018
 #define SFB_K7S3 0.433883739117558120476
+#define SFB_K9C1 0.766044443118978035202
+#define SFB_K9S1 0.642787609686539326323
+#define SFB_K9C2 0.173648177666930348852
+#define SFB_K9S2 0.984807753012208059367
+#define SFB_K9C4 -0.939692620785908384054
+#define SFB_K9S4 0.342020143325668733044
 #define SFB_K8 0.707106781186547524401
 #define SFB_K16C 0.923879532511286756128
 #define SFB_K16S 0.382683432365089771728
@@ -203,6 +209,62 @@ template <class T, class C> SFB_HD void bfly15(C* v) {
     }
 }
 
+// Radix A * B with coprime A and B as a prime-factor (Good-Thomas) DFT, as radix 15 above: input
+// n = (B*n1 + A*n2) mod AB, B-point DFTs over n2, A-point DFTs over n1, output k = (B*b*k1 + A*a*k2)
+// mod AB with b = B^-1 mod A and a = A^-1 mod B.
+template <int R, class T, class C> SFB_HD void dft(C* v);
+
+SFB_HD constexpr int inverse_mod(int a, int m) {
+    for (int x = 1; x < m; ++x)
+        if (a * x % m == 1) return x;
+    return 1;
+}
+
+template <int A, int B, class T, class C> SFB_HD void bfly_pfa(C* v) {
+    constexpr int R = A * B, kA = B * inverse_mod(B % A, A), kB = A * inverse_mod(A % B, B);
+    C a[A][B];
+#pragma unroll
+    for (int n1 = 0; n1 < A; ++n1) {
+#pragma unroll
+        for (int n2 = 0; n2 < B; ++n2) a[n1][n2] = v[(B * n1 + A * n2) % R];
+        dft<B, T>(a[n1]);
+    }
+#pragma unroll
+    for (int k2 = 0; k2 < B; ++k2) {
+        C b[A];
+#pragma unroll
+        for (int n1 = 0; n1 < A; ++n1) b[n1] = a[n1][k2];
+        dft<A, T>(b);
+#pragma unroll
+        for (int k1 = 0; k1 < A; ++k1) v[(kA * k1 + kB * k2) % R] = b[k1];
+    }
+}
+
+// Radix 9 as 3 x 3: n = n2 + 3*n1, three-point DFTs over n1, twiddles W9^(n2*k1), three-point
+// DFTs over n2; X[k1 + 3*k2].
+template <class T, class C> SFB_HD void bfly9(C* v) {
+    C a[3][3];
+#pragma unroll
+    for (int n2 = 0; n2 < 3; ++n2) {
+#pragma unroll
+        for (int n1 = 0; n1 < 3; ++n1) a[n2][n1] = v[n2 + 3 * n1];
+        bfly3<T>(a[n2]);
+    }
+    const C w1 = cmake<C>(T(SFB_K9C1), T(-SFB_K9S1)), w2 = cmake<C>(T(SFB_K9C2), T(-SFB_K9S2)),
+            w4 = cmake<C>(T(SFB_K9C4), T(-SFB_K9S4));
+    a[1][1] = cmul(a[1][1], w1);
+    a[1][2] = cmul(a[1][2], w2);
+    a[2][1] = cmul(a[2][1], w2);
+    a[2][2] = cmul(a[2][2], w4);
+#pragma unroll
+    for (int k1 = 0; k1 < 3; ++k1) {
+        C b[3] = {a[0][k1], a[1][k1], a[2][k1]};
+        bfly3<T>(b);
+#pragma unroll
+        for (int k2 = 0; k2 < 3; ++k2) v[k1 + 3 * k2] = b[k2];
+    }
+}
+
 // u[r] *= w^r for r = 1..R-1, the powers formed by a balanced product tree
 // (w^r = w^h * w^(r-h), h the largest power of two <= r): at most log2(R)+1 roundings deep.
 template <int R, class C> SFB_HD void twiddle_powers(C* u, C w) {
@@ -259,6 +321,16 @@ template <int R, class T, class C> SFB_HD void dft(C* v) {
         bfly7<T>(v);
     } else if constexpr (R == 8) {
         bfly8<T>(v);
+    } else if constexpr (R == 6) {
+        bfly_pfa<2, 3, T>(v);
+    } else if constexpr (R == 9) {
+        bfly9<T>(v);
+    } else if constexpr (R == 10) {
+        bfly_pfa<2, 5, T>(v);
+    } else if constexpr (R == 12) {
+        bfly_pfa<3, 4, T>(v);
+    } else if constexpr (R == 14) {
+        bfly_pfa<2, 7, T>(v);
     } else if constexpr (R == 15) {
         bfly15<T>(v);
     } else if constexpr (R == 16) {

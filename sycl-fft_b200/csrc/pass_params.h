@@ -28,6 +28,14 @@ namespace sfb {
 constexpr int kMaxStages = 16;
 
 enum : int { kModeK = 0, kModeC = 1 };         // thread mapping / coalesced dimension
+// Thread mappings of smooth_kernel.cuh, input side then output side: K lanes walk a line's elements
+// (element stride 1), C lanes walk adjacent lines (line stride 1).
+enum : int { kSmoothKK = 0, kSmoothCC = 1, kSmoothCK = 2, kSmoothKC = 3 };
+// Rows of a radix-R stage's twiddle table in smooth_kernel.cuh: W^(r*jm) for r = 1, 2, 4, 8 below R.
+#if defined(__CUDACC__)
+__host__ __device__
+#endif
+constexpr int smooth_tw_entries(int R) { return R > 8 ? 4 : R > 4 ? 3 : R > 2 ? 2 : 1; }
 enum : int { kSelNone = 0, kSelCol = 1, kSelOuterLo = 2, kSelColMod = 3 };
 
 struct LineLayout {

@@ -4,11 +4,13 @@
 #include "fixed_catalog.h"
 #include "fused4_catalog.h"
 #include "piped_catalog.h"
+#include "smooth_catalog.h"
 #include "tc_catalog.h"
 #include "bluestein_catalog.h"
 #include "tc_shape.h"
 
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <limits>
 #include <map>
@@ -400,6 +402,65 @@ struct Builder {
         ps.fixed_id = e->id;
         ps.fixed_feat = feat;
         use_base_table(ps);
+    }
+
+    // Stage twiddles of a smooth_catalog.h kernel: per stage the rows W_(ns*R)^(r*jm), jm < ns, for
+    // r = 1, 2, 4, 8 below R.
+    int smooth_table(const SmoothEntry& e) {
+        std::vector<int> key(e.radices, e.radices + e.nstages);
+        key.push_back(-2);  // distinct from the other table layouts of the radices
+        auto it = seq_tables.find(key);
+        if (it != seq_tables.end()) return it->second;
+        std::vector<int64_t> ckey(e.radices, e.radices + e.nstages);
+        ckey.push_back(-600);
+        auto tw = cached_table(ckey, [&] {
+            std::vector<std::complex<double>> t;
+            int64_t ns = 1;
+            for (int s = 0; s < e.nstages; ++s) {
+                const int R = e.radices[s];
+                for (int q = 0; q < smooth_tw_entries(R); ++q)
+                    for (int64_t jm = 0; jm < ns; ++jm) t.push_back(cis_neg((int64_t(1) << q) * jm, ns * R));
+                ns *= R;
+            }
+            return t;
+        });
+        const int id = add_table(*tw);
+        seq_tables[key] = id;
+        return id;
+    }
+
+    // The size-specialised kernel of this pass's length and thread mapping, where the catalog has one and
+    // the pass carries nothing but conjugations, a scale and the four-step twiddle.
+    void try_smooth(PassSpec& ps) {
+        const PassParams& p = ps.p;
+        if (ps.smooth_id >= 0 || req.no_fixed || req.force_maxv || req.force_w) return;
+        if (ps.tc_id >= 0 || ps.piped_id >= 0 || ps.cluster_id >= 0 || ps.blue_id >= 0 || ps.rader || ps.cluster_pipe ||
+            ps.tma || p.fft2.nstages > 0 || ps.tables.premul >= 0 || ps.tables.postmul >= 0 || ps.tables.pointwise >= 0)
+            return;
+        if (p.in.d != 1 || p.out.d != 1) return;
+        int kind;
+        const bool tw4 = p.tw4_sign != 0;
+        if (p.mode == kModeC) {
+            if (p.in.cs != 1 || p.out.cs != 1) return;
+            if (tw4 ? p.sel_mode != kSelCol || p.g_k != p.n_cols || p.n * p.g_k > (int64_t(1) << 30)
+                    : p.sel_mode != kSelNone || p.in_len < p.n || p.out_len < p.n)
+                return;
+            kind = kSmoothCC;
+        } else {
+            if (tw4 || p.sel_mode != kSelNone || p.in.ks != 1 || p.in_len < p.n || p.out_len < p.n) return;
+            if (p.ts_rows > 0 || p.store_via_smem) {  // row pass of a contiguous four-step, stored transposed
+                if (p.ts_rows == 0 && p.out.cs != 1) return;
+                if (p.ts_rows > 0 && p.n_cols % p.ts_rows != 0) return;
+                kind = kSmoothKC;
+            } else {
+                if (p.out.ks != 1 || p.n_outer != 1) return;
+                kind = kSmoothKK;
+            }
+        }
+        const SmoothEntry* e = find_smooth(req.dbl, kind, tw4, p.n);
+        if (!e || static_cast<int64_t>(e->w) * e->pitch * cs > smem_limit) return;
+        ps.tables.smooth = smooth_table(*e);
+        ps.smooth_id = e->id;
     }
 
     bool fits(int64_t n, int mode) {
@@ -1549,6 +1610,34 @@ const FixedEntry* find_fixed(bool dbl, int mode, int n, int feat) {
     return nullptr;
 }
 
+namespace {
+const std::vector<SmoothEntry>& smooth_entries() {
+    static const std::vector<SmoothEntry> all = {
+#define SFB_X(ID, DBL, KIND, TW4, N, TPL, W, PADS, PITCH, MAXT, MINB, ...) \
+    {ID, DBL, KIND, TW4, N, TPL, W, PADS, PITCH, MAXT, MINB, {__VA_ARGS__}, count_args(__VA_ARGS__)},
+        SFB_SMOOTH_CATALOG(SFB_X)
+#undef SFB_X
+    };
+    return all;
+}
+}  // namespace
+
+const SmoothEntry* find_smooth(bool dbl, int kind, bool tw4, int n) {
+    static const std::map<std::array<int, 4>, const SmoothEntry*> index = [] {
+        std::map<std::array<int, 4>, const SmoothEntry*> m;
+        for (const SmoothEntry& e : smooth_entries()) m[{e.dbl, e.kind, e.tw4, e.n}] = &e;
+        return m;
+    }();
+    const auto it = index.find({dbl ? 1 : 0, kind, tw4 ? 1 : 0, n});
+    return it == index.end() ? nullptr : it->second;
+}
+
+// Ids number the entries in catalog order.
+const SmoothEntry* smooth_entry(int id) {
+    const auto& all = smooth_entries();
+    return id >= 0 && id < static_cast<int>(all.size()) ? &all[id] : nullptr;
+}
+
 // Runtime-length passes whose layout the contiguous kernel (lean_kernel.cuh) covers: whole
 // contiguous lines, or the column / row pass of a contiguous four-step, with no table,
 // padding or second FFT, at least two stages in the radix order 16, 8, 4, 2, 3, 5, 7 and a
@@ -1647,6 +1736,7 @@ PlanSpec make_plan(const PlanRequest& req) {
     if (plan.passes.empty()) b.copy_pass(cur);
     plan.passes.back().p.scale = plan.scale;
     for (auto& ps : plan.passes) {
+        b.try_smooth(ps);
         mark_lean(ps, req.dbl ? 16 : 8);
         if (!ps.lean) continue;
         const std::vector<int> r = lean_radix15(ps);
@@ -1681,7 +1771,11 @@ std::string describe_plan(const PlanSpec& plan) {
            << ",\"dst\":" << int(ps.dst) << ",\"bytes\":" << ps.bytes_moved
            << ",\"store_via_smem\":" << p.store_via_smem << ",\"fixed_id\":" << ps.fixed_id
            << ",\"piped_id\":" << ps.piped_id << ",\"tc_id\":" << ps.tc_id << ",\"blue_id\":" << ps.blue_id << ",\"tma\":" << (ps.tma ? 1 : 0) << ",\"cluster_id\":" << ps.cluster_id << ",\"cluster_pipe\":" << (ps.cluster_pipe ? 1 : 0) << ",\"cluster\":[" << ps.cl_n1 << "," << ps.cl_n2 << ","
-           << ps.cl_p << "],\"rader\":" << (ps.rader ? 1 : 0) << ",\"lean\":" << (ps.lean ? 1 : 0) << "}";
+           << ps.cl_p << "],\"rader\":" << (ps.rader ? 1 : 0) << ",\"lean\":" << (ps.lean ? 1 : 0)
+           << ",\"smooth_id\":" << ps.smooth_id << ",\"smooth_radices\":[";
+        if (const SmoothEntry* e = smooth_entry(ps.smooth_id))
+            for (int s = 0; s < e->nstages; ++s) os << (s ? "," : "") << e->radices[s];
+        os << "]}";
     }
     os << "]}";
     return os.str();

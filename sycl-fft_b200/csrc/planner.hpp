@@ -36,6 +36,7 @@ struct TableIds {
     int tc_tw = -1;  // two-level W_N^k table of the tensor-core kernel
     int cl_base = -1;  // base twiddles of the pipelined cluster kernel's 256-point FFTs
     int perm_in = -1, perm_out = -1;  // Rader permutations (PlanSpec::index_tables)
+    int smooth = -1;  // stage twiddles of the smooth_catalog.h kernel
 };
 
 struct KernelChoice {
@@ -79,6 +80,9 @@ struct PassSpec {
     // (tw_base), so it only runs on the lean kernel.
     bool lean = false;
     int lean_feat = 0;
+    // size-specialised kernel of the 7-smooth lengths (smooth_catalog.h) that runs this pass in place of
+    // the kernel named above, with its own stage sequence (table tables.smooth); -1: none
+    int smooth_id = -1;
 };
 
 // The lean kernel's instantiations (lean_variants.cu): float with 16 values per thread, double
@@ -108,6 +112,16 @@ struct FixedEntry {
 const FixedEntry* find_fixed(bool dbl, int mode, int n, int feat);
 // A fused four-step kernel (fused4_catalog.h) runs these column and row entries together.
 bool has_fused4(bool dbl, int col_id, int row_id);
+
+// One entry of smooth_catalog.h as seen by the host. kind: kSmoothKK / CC / CK / KC, the lane mappings of the
+// input and output sides (smooth_kernel.cuh).
+struct SmoothEntry {
+    int id, dbl, kind, tw4, n, tpl, w, pads, pitch, maxt, minb;
+    int radices[kMaxStages];
+    int nstages;
+};
+const SmoothEntry* find_smooth(bool dbl, int kind, bool tw4, int n);
+const SmoothEntry* smooth_entry(int id);
 
 // One entry of piped_catalog.h as seen by the host.
 struct PipedEntry {

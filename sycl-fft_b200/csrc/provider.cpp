@@ -27,6 +27,7 @@
 #include "fixed_launch.hpp"
 #include "launch.hpp"
 #include "lean_launch.hpp"
+#include "smooth_launch.hpp"
 #include "piped_launch.hpp"
 #include "tc_launch.hpp"
 #include "tma_launch.hpp"
@@ -89,6 +90,8 @@ struct BoundPass {
     // Bluestein forward column pass whose row and inverse column passes (the next two) can run
     // with it in one fused launch, or nullptr
     const FusedBlueEntry* fusedblue = nullptr;
+    const SmoothEntry* smooth = nullptr;  // size-specialised kernel of a 7-smooth length, and its twiddles
+    const void* smooth_tw = nullptr;
 };
 
 TcParams to_tc(const PassParams& p, const void* tw, int* status) {
@@ -506,11 +509,22 @@ DevicePlan* build_plan(PlanRequest req, int device, uint32_t flags, const std::s
 
     // All tables in one allocation, each 256-byte aligned: the complex tables (cast to the
     // plan precision), then the int32 index tables.
+    // A pass on a smooth_catalog.h kernel reads that kernel's stage table instead of tw1 (unless the fused
+    // multi-pass kernels, an opt-in, take it): tables no kernel reads are not uploaded.
+    const char* f4env = std::getenv("SYCLFFT_B200_FUSED4");
+    const bool fused_opt_in = f4env && f4env[0] == '1';
+    std::vector<char> read(plan->spec.tables.size(), fused_opt_in ? 1 : 0);
+    for (const PassSpec& ps : plan->spec.passes) {
+        const TableIds& t = ps.tables;
+        for (int id : {ps.smooth_id >= 0 ? -1 : t.tw1, t.tw2, t.premul, t.pointwise, t.postmul, t.tw4_hi, t.tw4_lo, t.tc_tw,
+                       t.cl_base, t.smooth})
+            if (id >= 0) read[id] = 1;
+    }
     std::vector<size_t> offsets(plan->spec.tables.size()), ioffsets(plan->spec.index_tables.size());
     size_t total = 0;
     for (size_t i = 0; i < plan->spec.tables.size(); ++i) {
         offsets[i] = total;
-        total += (plan->spec.table_sizes[i] * cs + 255) / 256 * 256;
+        if (read[i]) total += (plan->spec.table_sizes[i] * cs + 255) / 256 * 256;
     }
     for (size_t i = 0; i < plan->spec.index_tables.size(); ++i) {
         ioffsets[i] = total;
@@ -522,6 +536,7 @@ DevicePlan* build_plan(PlanRequest req, int device, uint32_t flags, const std::s
     UploadStaging::Buffer* blob = staging.acquire(table_bytes);
     std::memset(blob->data, 0, table_bytes);
     for (size_t i = 0; i < plan->spec.tables.size(); ++i) {
+        if (!read[i]) continue;
         if (req.dbl) pack_table<double>(plan->spec.tables[i], blob->data, offsets[i]);
         else pack_table<float>(plan->spec.tables[i], blob->data, offsets[i]);
     }
@@ -575,7 +590,7 @@ DevicePlan* build_plan(PlanRequest req, int device, uint32_t flags, const std::s
     if (flags & SYCLFFT_B200_CREATE_SYNC) check(cudaStreamSynchronize(ms), "plan tables");
 
     auto tab = [&](int id) -> const void* {
-        return id < 0 ? nullptr : static_cast<const unsigned char*>(plan->table_mem) + offsets[id];
+        return id < 0 || !read[id] ? nullptr : static_cast<const unsigned char*>(plan->table_mem) + offsets[id];
     };
     for (const PassSpec& ps : plan->spec.passes) {
         if (ps.fixed_id < 0 && ps.cluster_id < 0 && ps.tc_id < 0 && ps.blue_id < 0 && !has_variant(req.dbl, ps.kc.maxv, ps.kc.maxt))
@@ -612,6 +627,8 @@ DevicePlan* build_plan(PlanRequest req, int device, uint32_t flags, const std::s
         }
         bp.pp = to_piped(bp.p, plan->status);
         bp.tp = to_tc(bp.p, tab(ps.tables.tc_tw), plan->status);
+        bp.smooth = smooth_entry(ps.smooth_id);
+        bp.smooth_tw = tab(ps.tables.smooth);
         plan->passes.push_back(bp);
     }
     // four-step column + row passes (and Bluestein's three passes) of a contiguous axis with a
@@ -1142,11 +1159,46 @@ LeanParams to_lean(const PassParams& p) {
     return L;
 }
 
+// A pass on its smooth_catalog.h kernel.
+SmoothParams to_smooth(const PassParams& p, const void* tw, int64_t* n_outer) {
+    SmoothParams s;
+    s.n_cols = p.n_cols;
+    *n_outer = p.n_outer;
+    s.in_hi = p.in.hi;
+    s.in_cs = p.in.cs;
+    s.in_ks = p.in.ks;
+    s.out_hi = p.out.hi;
+    s.out_cs = p.out.cs;
+    s.out_ks = p.out.ks;
+    if (p.ts_rows > 0) {
+        // the flat rows o * ts_rows + k1 of the size-specialised four-step row pass
+        s.n_cols = p.ts_rows;
+        *n_outer = p.n_cols / p.ts_rows;
+        s.in_hi = p.ts_rows * p.in.cs;
+        s.out_hi = p.ts_line;
+        s.out_cs = 1;
+        s.out_ks = p.ts_rows;
+    }
+    s.tw = tw;
+    s.conj_in = p.conj_in;
+    s.conj_out = p.conj_out;
+    s.scale = p.scale;
+    s.tw4_hi = p.tw4_hi;
+    s.tw4_lo = p.tw4_lo;
+    s.tw4_shift = p.tw4_shift;
+    s.tw4_conj = p.tw4_sign > 0 ? 1 : 0;
+    return s;
+}
+
 // Launches one bound pass of a plan on its kernel family.
 void launch_bound_pass(DevicePlan* plan, const BoundPass& bp, void* src, void* dst, cudaStream_t stream) {
     const bool aligned = (reinterpret_cast<uintptr_t>(src) % 16 == 0) && (reinterpret_cast<uintptr_t>(dst) % 16 == 0);
     const PassSpec& ps = bp.spec_ref();
-    if (ps.blue_id >= 0) {
+    if (bp.smooth) {
+        int64_t n_outer = 1;
+        const SmoothParams sp = to_smooth(bp.p, bp.smooth_tw, &n_outer);
+        check(launch_smooth(*bp.smooth, sp, n_outer, plan->sms, src, dst, stream), "FFT pass launch");
+    } else if (ps.blue_id >= 0) {
         check(launch_blue(ps.blue_id, plan->spec.req.dbl, ps.blue_kind, ps.rader, bp.fp, ps.threads,
                           static_cast<size_t>(ps.smem_bytes), bp.p.tiles, src, dst, stream),
               "FFT Bluestein pass launch");

@@ -19,8 +19,13 @@ static int dispatch(int radix, const T* in, T* out) {
         case 3: run<3, T>(in, out); return 0;
         case 4: run<4, T>(in, out); return 0;
         case 5: run<5, T>(in, out); return 0;
+        case 6: run<6, T>(in, out); return 0;
         case 7: run<7, T>(in, out); return 0;
         case 8: run<8, T>(in, out); return 0;
+        case 9: run<9, T>(in, out); return 0;
+        case 10: run<10, T>(in, out); return 0;
+        case 12: run<12, T>(in, out); return 0;
+        case 14: run<14, T>(in, out); return 0;
         case 15: run<15, T>(in, out); return 0;
         case 16: run<16, T>(in, out); return 0;
         default: return 1;

@@ -101,3 +101,20 @@ def primitive_root(p):
     L.emu_primitive_root.restype = ctypes.c_uint64
     L.emu_primitive_root.argtypes = [ctypes.c_uint64]
     return int(L.emu_primitive_root(int(p)))
+
+
+def smooth_run(x, shape, batch, direction, norm=0, double=False, in_place=False, w_lines=0):
+    """A contiguous plan stepped through the 7-smooth kernels' index arithmetic; None when a pass of the
+    plan is not one of them."""
+    L = _load("libsmooth_check.so")
+    L.smooth_run.argtypes = [ctypes.c_int] * 4 + [ctypes.c_uint, ctypes.c_void_p, ctypes.c_uint64, ctypes.c_int,
+                                                  ctypes.c_void_p, ctypes.c_void_p, ctypes.c_char_p, ctypes.c_size_t]
+    sh = (ctypes.c_uint64 * 3)(*(list(shape) + [0] * (3 - len(shape))))
+    xin = np.ascontiguousarray(np.asarray(x, dtype=np.complex128))
+    out = np.zeros_like(xin)
+    err = ctypes.create_string_buffer(1024)
+    rc = L.smooth_run(int(double), int(direction), int(norm), int(in_place), len(shape), sh, int(batch), int(w_lines),
+                      xin.ctypes.data, out.ctypes.data, err, 1024)
+    if rc == 1:
+        raise RuntimeError(err.value.decode())
+    return None if rc == 2 else out

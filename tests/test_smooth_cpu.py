@@ -1,0 +1,77 @@
+"""Host checks of the size-specialised kernels of the 7-smooth lengths: every catalog entry's geometry, their
+additional butterflies, and plans stepped thread by thread through the kernel's index arithmetic (bounds,
+shared-memory races, twiddle rows, strides) against numpy's FP64 FFT."""
+import os
+import re
+
+import numpy as np
+import pytest
+
+from conftest import fp64_fft, gaussian_complex, norm_scale, rel_l2
+from native_libs import butterfly, describe, smooth_run
+
+KK, CC, CK, KC = 0, 1, 2, 3
+
+
+def catalog():
+    src = open(os.path.join(os.path.dirname(__file__), "..", "sycl-fft_b200", "csrc", "smooth_catalog.h")).read()
+    return [tuple(int(v) for v in m.split(",")) for m in re.findall(r"X\(([-0-9, ]+)\)", src)]
+
+
+@pytest.mark.parametrize("radix", [6, 9, 10, 12, 14])
+def test_composite_butterflies(radix):
+    x = gaussian_complex(radix, radix, np.complex128)
+    assert np.max(np.abs(butterfly(radix, x) - np.fft.fft(x))) < 1e-14 * radix
+    assert np.max(np.abs(butterfly(radix, x, double=False) - np.fft.fft(x))) < 2e-6 * radix
+
+
+def test_catalog_geometry():
+    """Ids number the entries; radices multiply to the length; lines fit the block, the registers of an
+    SM and its shared memory; the padded row holds the line; mappings with a column side take a power of
+    two of lines."""
+    entries = catalog()
+    assert [e[0] for e in entries] == list(range(len(entries)))
+    assert len({(e[1], e[2], e[3], e[4]) for e in entries}) == len(entries)
+    for e in entries:
+        _, dbl, kind, tw4, n, tpl, w, pads, pitch, maxt, minb, *radices = e
+        assert np.prod(radices) == n and len(radices) >= 2 and max(radices) <= 16, e
+        assert (w * tpl + 31) // 32 * 32 == maxt <= 1024 and maxt * minb <= 2048, e
+        assert pitch > (n - 1) + ((n - 1) >> pads if pads else 0), e
+        assert w * pitch * (16 if dbl else 8) <= 227 * 1024, e
+        assert kind == KK or w & (w - 1) == 0, e
+        assert not tw4 or kind == CC, e
+
+
+# the shortest and longest lines of each mapping, one with idle threads in a stage, several lines per block
+@pytest.mark.parametrize("double", [False, True])
+@pytest.mark.parametrize("shape,batch", [([18], 70), ([45], 97), ([105], 25), ([810], 3), ([1029], 2), ([3000], 2),
+                                         ([6125], 1), ([16807], 1), ([30000], 1), ([65536], 1), ([36, 40], 2),
+                                         ([343, 48], 1), ([15, 20, 18], 2), ([25, 2025], 1)], ids=str)
+def test_contiguous_plans_by_thread(shape, batch, double):
+    n = int(np.prod(shape))
+    x = gaussian_complex(n * batch, n + batch, np.complex128)
+    for d, norm, ip in ((-1, 3, False), (1, 2, True)):
+        y = smooth_run(x, shape, batch, d, norm, double, ip)
+        if y is None:
+            pytest.skip("a pass of this plan is not a 7-smooth kernel")
+        assert rel_l2(y, fp64_fft(x, shape, batch, d, norm_scale(norm, d, n))) < 1e-13
+
+
+@pytest.mark.parametrize("w_lines", [1, 2, 3])
+def test_fewer_lines_per_block(w_lines):
+    x = gaussian_complex(100 * 7, 3, np.complex128)
+    y = smooth_run(x, [100], 7, -1, w_lines=w_lines)
+    assert rel_l2(y, fp64_fft(x, [100], 7, -1)) < 1e-13
+
+
+def test_dispatch():
+    """Where a plan takes a 7-smooth kernel: whole lines, strided axes and both passes of a four-step;
+    not the generic or tensor-core plans, nor passes with Bluestein tables."""
+    def ids(shape, **kw):
+        return [p["smooth_id"] >= 0 for p in describe(shape, 4, **kw)["passes"]]
+
+    assert ids([3000]) == [True]
+    assert ids([680400]) == [True, True]
+    assert ids([840, 1200]) == [True, True]
+    assert ids([256, 256], split_bf16=True) == [False, False]
+    assert ids([1009]) == [False]
