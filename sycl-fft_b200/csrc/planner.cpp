@@ -1332,6 +1332,37 @@ struct Builder {
         cur = Buf::Output;
     }
 
+    // One pass over strided lines (PlanRequest::strided_line): the layout change happens in the pass's own
+    // loads and stores.
+    void line_pass(Buf& cur) {
+        const int64_t n = static_cast<int64_t>(req.shape[0]);
+        const int kind = strided_line_kind(req.line_in, req.line_out);
+        const SmoothEntry* e = kind < 0 || n > (1 << 20) ? nullptr : find_smooth(req.dbl, kind, false, static_cast<int>(n));
+        if (!e || static_cast<int64_t>(e->w) * e->pitch * cs > smem_limit)
+            throw std::runtime_error("no single-pass kernel for this strided length");
+        PassSpec ps;
+        ps.kind = "single";
+        PassParams& p = ps.p;
+        p.n = static_cast<int>(n);
+        p.mode = kind == kSmoothKK || kind == kSmoothKC ? kModeK : kModeC;
+        p.n_outer = 1;
+        p.n_cols = static_cast<int64_t>(req.batch);
+        p.in = req.line_in;
+        p.out = req.line_out;
+        p.in_len = p.out_len = n;
+        p.conj_in = p.conj_out = req.direction == 1;
+        SingleCfg cfg = single_cfg(n, req.dbl, 0);
+        set_fft(ps, p.fft1, &ps.tables.tw1, p.n, cfg);
+        geometry(ps, cfg, 1);
+        ps.tables.smooth = smooth_table(*e);
+        ps.smooth_id = e->id;
+        ps.src = cur;
+        ps.dst = Buf::Output;
+        ps.bytes_moved = 2 * static_cast<int64_t>(plan.elements) * cs;
+        plan.passes.push_back(ps);
+        cur = Buf::Output;
+    }
+
     void copy_pass(Buf& cur) {
         PassSpec ps;
         ps.kind = "copy";
@@ -1632,6 +1663,12 @@ const SmoothEntry* find_smooth(bool dbl, int kind, bool tw4, int n) {
     return it == index.end() ? nullptr : it->second;
 }
 
+int strided_line_kind(const LineLayout& in, const LineLayout& out) {
+    const bool kin = in.ks == 1, kout = out.ks == 1;
+    if ((!kin && in.cs != 1) || (!kout && out.cs != 1)) return -1;
+    return kin ? (kout ? kSmoothKK : kSmoothKC) : (kout ? kSmoothCK : kSmoothCC);
+}
+
 // Ids number the entries in catalog order.
 const SmoothEntry* smooth_entry(int id) {
     const auto& all = smooth_entries();
@@ -1726,7 +1763,11 @@ PlanSpec make_plan(const PlanRequest& req) {
     Buf cur = Buf::Input;
     const int rank = static_cast<int>(req.shape.size());
     const int64_t E = static_cast<int64_t>(plan.elements);
-    for (int ax = rank - 1; ax >= 0; --ax) {
+    if (req.strided_line) {
+        if (rank != 1) throw std::invalid_argument("strided lines are one-dimensional");
+        b.line_pass(cur);
+    }
+    for (int ax = rank - 1; ax >= 0 && !req.strided_line; --ax) {
         const int64_t L = static_cast<int64_t>(req.shape[ax]);
         if (L == 1 || ((req.skip_axes >> ax) & 1u)) continue;
         int64_t s = 1;

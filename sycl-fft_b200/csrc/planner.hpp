@@ -122,6 +122,9 @@ struct SmoothEntry {
 };
 const SmoothEntry* find_smooth(bool dbl, int kind, bool tw4, int n);
 const SmoothEntry* smooth_entry(int id);
+// The mapping pair of a strided one-dimensional layout, or -1 when a side is neither contiguous lines nor
+// adjacent columns.
+int strided_line_kind(const LineLayout& in, const LineLayout& out);
 
 // One entry of piped_catalog.h as seen by the host.
 struct PipedEntry {
@@ -181,6 +184,11 @@ struct PlanRequest {
     // complex<double> 65536-point lines: the cluster pass (cluster_p = 16) on the pipelined
     // cluster kernel (opt-in)
     bool cluster_pipe = false;
+    // One-dimensional transforms of strided lines in one pass: line c's element k at c * cs + k * ks of
+    // each side (ks == 1: contiguous lines, cs == 1: adjacent columns). Only for lengths with a
+    // smooth_catalog.h kernel of the two mappings (strided_line_kind).
+    bool strided_line = false;
+    LineLayout line_in, line_out;
     // prime lengths L take Bluestein's convolution even where the catalog covers L - 1 (Rader)
     bool no_rader = false;
 };

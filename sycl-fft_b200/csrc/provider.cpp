@@ -271,6 +271,7 @@ struct DevicePlan {
     bool strided = false;
     Layout in_layout, out_layout;
     bool in_contig = true, out_contig = true;
+    bool direct = false;            // `inner` reads and writes the layouts itself (one pass, one-dimensional)
     bool interleaved = false;       // both sides the dense [L.., batch] array: `inner` runs on it directly
     void* pack_buf = nullptr;       // contiguous batch x prod(L) complex
 
@@ -410,7 +411,8 @@ void pack_table(const std::vector<std::complex<double>>& t, unsigned char* blob,
     }
 }
 
-DevicePlan* create_plan(const syclfft_b200_plan_config_v1& cfg, uint32_t flags = 0, uint32_t skip_axes = 0);
+DevicePlan* create_plan(const syclfft_b200_plan_config_v1& cfg, uint32_t flags = 0, uint32_t skip_axes = 0,
+                        const LineLayout* line_in = nullptr, const LineLayout* line_out = nullptr);
 void execute_plan(DevicePlan* plan, const void* in, void* out, cudaStream_t stream, uint64_t batch = 0,
                   int direction = 0, int normalization = -1);
 
@@ -438,7 +440,8 @@ DevicePlan* spectrum_plan(int device, int64_t M) {
 DevicePlan* build_plan(PlanRequest req, int device, uint32_t flags, const std::string& tuning);
 PlanRequest tune(const PlanRequest& req, int device, std::string* report);
 
-DevicePlan* create_plan(const syclfft_b200_plan_config_v1& cfg, uint32_t flags, uint32_t skip_axes) {
+DevicePlan* create_plan(const syclfft_b200_plan_config_v1& cfg, uint32_t flags, uint32_t skip_axes,
+                        const LineLayout* line_in, const LineLayout* line_out) {
     if (cfg.abi_version != SYCLFFT_B200_PROVIDER_ABI_VERSION) throw std::runtime_error("B200 provider ABI mismatch");
     if (cfg.scalar != SYCLFFT_B200_SCALAR_FLOAT && cfg.scalar != SYCLFFT_B200_SCALAR_DOUBLE)
         throw std::invalid_argument("unsupported scalar type");
@@ -452,6 +455,11 @@ DevicePlan* create_plan(const syclfft_b200_plan_config_v1& cfg, uint32_t flags, 
     req.batch = cfg.batch_count;
     req.split_bf16 = !req.dbl && (flags & SYCLFFT_B200_CREATE_SPLIT_BF16) != 0;
     req.skip_axes = skip_axes;
+    if (line_in && line_out) {
+        req.strided_line = true;
+        req.line_in = *line_in;
+        req.line_out = *line_out;
+    }
     // SYCLFFT_B200_KERNELS=generic: plan every pass on the runtime-parameterised kernel
     // (used to test and compare it against the size-specialised kernels).
     if (const char* k = std::getenv("SYCLFFT_B200_KERNELS")) req.no_fixed = std::strcmp(k, "generic") == 0;
@@ -486,7 +494,7 @@ DevicePlan* create_plan(const syclfft_b200_plan_config_v1& cfg, uint32_t flags, 
     if (device < 0) check(cudaGetDevice(&device), "cudaGetDevice");
     DeviceGuard guard(device);
     std::string tuning;
-    if (cfg.measure) {
+    if (cfg.measure && !req.strided_line) {
         // planning_mode::measure: time the candidate decompositions and kernels
         (void)make_plan(req);  // argument validation before any device work
         req = tune(req, device, &tuning);
@@ -967,6 +975,42 @@ DevicePlan* create_strided_plan(const syclfft_b200_plan_config_v1& cfg, const sy
         plan->inner = std::move(inner);
         return plan.release();
     }
+    if (cfg.rank == 1) {
+        // Lines whose sides are each contiguous lines or adjacent columns: where the length has a
+        // smooth_catalog.h kernel of those mappings it reads and writes the layouts itself, one HBM pass
+        // instead of two or three (1024 points x 65536, float, columns -> rows: 397 -> 239 us;
+        // 177 lengths of 64 MB matrices 2.4 to 2.7x).
+        LineLayout li, lo;
+        li.cs = in.dist;
+        li.ks = in.len[0] > 1 ? in.stride[0] : 1;
+        lo.cs = out.dist;
+        lo.ks = out.len[0] > 1 ? out.stride[0] : 1;
+        const bool dbl = cfg.scalar == SYCLFFT_B200_SCALAR_DOUBLE;
+        const bool split = !dbl && (flags & SYCLFFT_B200_CREATE_SPLIT_BF16) != 0;
+        const char* generic = std::getenv("SYCLFFT_B200_KERNELS");
+        const int kind = strided_line_kind(li, lo);
+        if (kind >= 0 && !split && !(generic && std::strcmp(generic, "generic") == 0) && cfg.lengths[0] <= (1u << 20) &&
+            find_smooth(dbl, kind, false, static_cast<int>(cfg.lengths[0]))) {
+            std::unique_ptr<DevicePlan> inner(create_plan(cfg, flags | SYCLFFT_B200_CREATE_SYNC, 0, &li, &lo));
+            auto plan = std::make_unique<DevicePlan>();
+            plan->device = inner->device;
+            plan->sms = inner->sms;
+            plan->spec.req = inner->spec.req;
+            plan->spec.transform_size = inner->spec.transform_size;
+            plan->spec.elements = inner->spec.elements;
+            plan->status = inner->status;
+            plan->strided = true;
+            plan->direct = true;
+            plan->in_layout = in;
+            plan->out_layout = out;
+            plan->in_contig = ic;
+            plan->out_contig = oc;
+            DeviceGuard guard(plan->device);
+            check(cudaEventCreateWithFlags(&plan->done, cudaEventDisableTiming), "cudaEventCreate");
+            plan->inner = std::move(inner);
+            return plan.release();
+        }
+    }
     syclfft_b200_plan_config_v1 c = cfg;
     c.in_place = (!ic && !oc) ? 1 : 0;  // both strided: transform the gathered copy in place
     std::unique_ptr<DevicePlan> inner(create_plan(c, flags | SYCLFFT_B200_CREATE_SYNC));
@@ -1010,7 +1054,9 @@ void execute_strided(DevicePlan* plan, const void* in, void* out, cudaStream_t s
     Layout li = plan->in_layout, lo = plan->out_layout;
     li.batch = lo.batch = static_cast<int64_t>(batch);
     DevicePlan* inner = plan->inner.get();
-    if (plan->interleaved) {
+    if (plan->direct) {
+        execute_plan(inner, in, out, stream, batch, direction, normalization);
+    } else if (plan->interleaved) {
         if (batch != planned)
             throw std::invalid_argument("a plan over an interleaved batch (distance 1) runs its whole batch");
         execute_plan(inner, in, out, stream, 0, direction, normalization);
@@ -1753,7 +1799,7 @@ SYCLFFT_B200_EXPORT int syclfft_b200_describe_plan(const void* plan, char* buf, 
         };
         s = "{\"layout\":{\"in\":" + side(p->in_layout, p->in_contig) + ",\"out\":" +
             side(p->out_layout, p->out_contig) + ",\"interleaved\":" + (p->interleaved ? "1" : "0") +
-            "},\"inner\":" + sfb::describe_plan(p->inner->spec) + "}";
+            ",\"direct\":" + (p->direct ? "1" : "0") + "},\"inner\":" + sfb::describe_plan(p->inner->spec) + "}";
     } else {
         s = sfb::describe_plan(p->spec);
         int fused = 0, fusedblue = 0;
@@ -1791,7 +1837,7 @@ SYCLFFT_B200_EXPORT int syclfft_b200_plan_launches(const void* plan) {
     if (p->real_kind) return p->real_fused ? 1 : sfb::pass_launches(p->inner.get()) + 1;
     if (p->strided)
         return sfb::pass_launches(p->inner.get()) +
-               (p->interleaved ? 0 : (p->in_contig ? 0 : 1) + (p->out_contig ? 0 : 1));
+               (p->interleaved || p->direct ? 0 : (p->in_contig ? 0 : 1) + (p->out_contig ? 0 : 1));
     return sfb::pass_launches(p);
 }
 

@@ -188,3 +188,21 @@ extern "C" int smooth_run(int dbl, int dir, int norm, int in_place, unsigned ran
     for (unsigned k = 0; k < rank; ++k) n *= static_cast<int64_t>(shape[k]);
     return run_plan(req, in, n, out, n, w_lines, err, cap);
 }
+
+// A strided one-dimensional plan (PlanRequest::strided_line).
+extern "C" int smooth_run_line(int dbl, int dir, int norm, int in_place, uint64_t n, uint64_t batch, const int64_t* cs_ks,
+                               const double* in, int64_t in_len, double* out, int64_t out_len, char* err, size_t cap) {
+    PlanRequest req;
+    req.dbl = dbl != 0;
+    req.direction = dir;
+    req.normalization = norm;
+    req.in_place = in_place != 0;
+    req.shape = {n};
+    req.batch = batch;
+    req.strided_line = true;
+    req.line_in.cs = cs_ks[0];
+    req.line_in.ks = cs_ks[1];
+    req.line_out.cs = cs_ks[2];
+    req.line_out.ks = cs_ks[3];
+    return run_plan(req, in, in_len, out, out_len, 0, err, cap);
+}

@@ -118,3 +118,21 @@ def smooth_run(x, shape, batch, direction, norm=0, double=False, in_place=False,
     if rc == 1:
         raise RuntimeError(err.value.decode())
     return None if rc == 2 else out
+
+
+def smooth_run_line(x, n, batch, layout, out, direction, norm=0, double=False, in_place=False):
+    """A strided one-dimensional plan (layout: (in cs, in ks, out cs, out ks)) likewise; writes into a copy
+    of `out`."""
+    L = _load("libsmooth_check.so")
+    L.smooth_run_line.argtypes = [ctypes.c_int] * 4 + [ctypes.c_uint64, ctypes.c_uint64, ctypes.c_void_p, ctypes.c_void_p,
+                                                       ctypes.c_int64, ctypes.c_void_p, ctypes.c_int64, ctypes.c_char_p,
+                                                       ctypes.c_size_t]
+    lay = (ctypes.c_int64 * 4)(*layout)
+    xin = np.ascontiguousarray(np.asarray(x, dtype=np.complex128))
+    got = np.array(out, dtype=np.complex128)
+    err = ctypes.create_string_buffer(1024)
+    rc = L.smooth_run_line(int(double), int(direction), int(norm), int(in_place), int(n), int(batch), lay,
+                           xin.ctypes.data, xin.size, got.ctypes.data, got.size, err, 1024)
+    if rc:
+        raise RuntimeError(err.value.decode() or "no single-pass kernel")
+    return got

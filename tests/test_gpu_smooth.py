@@ -1,6 +1,6 @@
 """GPU parity of the size-specialised kernels of the 7-smooth lengths (smooth_kernel.cuh): the shortest and
-longest lines of each thread mapping and lines per block cut off by the batch, against FP64 FFTs at the
-complex tolerance of the length (rel-L2 <= 1e-5 * log2 N float, 1e-12 * log2 N double)."""
+longest lines of each thread mapping, lines per block cut off by the batch, and strided layouts, against
+FP64 FFTs at the complex tolerance of the length (rel-L2 <= 1e-5 * log2 N float, 1e-12 * log2 N double)."""
 import numpy as np
 import pytest
 
@@ -44,3 +44,35 @@ def test_contiguous(sf, torch, shape, batch, dbl):
         o = a if in_place else torch.full_like(a, 9.0)
         (p.execute(a) if in_place else p.execute(a, o)).synchronize()
         assert rel_l2(o.cpu().numpy(), fp64_fft(x, shape, batch, d, norm_scale(norm, d, n))) <= tol(n, dbl)
+
+
+@pytest.mark.parametrize("dbl", [False, True], ids=["float", "double"])
+@pytest.mark.parametrize("n,b,src,dst", [
+    (64, 24, (1, 24), (64, 1)), (64, 1, (1, 5), (64, 1)), (60, 7, (1, 9), (1, 11)), (100, 5, (107, 1), (103, 1)),
+    (2048, 3, (1, 3), (2050, 1)), (1000, 17, (1001, 1), (1, 17)), (24, 33, (1, 2), (24, 1)), (1500, 9, (1, 9), (1500, 1)),
+    (1920, 130, (1, 131), (1, 130)),
+], ids=str)
+def test_strided_lines(sf, torch, n, b, src, dst, dbl):
+    """One launch for lines whose sides are contiguous (of any pitch) or adjacent columns; partial batches;
+    nothing outside the output layout is written."""
+    import ctypes
+    from syclfft_b200 import _provider
+    at_in = np.arange(b)[:, None] * src[0] + np.arange(n)[None, :] * src[1]
+    at_out = np.arange(b)[:, None] * dst[0] + np.arange(n)[None, :] * dst[1]
+    x = uniform_complex(int(at_in.max()) + 1, n + b, np.complex128 if dbl else np.complex64)
+    lay = sf.data_layout((src[1],), src[0], (dst[1],), dst[0])
+    p = sf.plan_many_dft("double" if dbl else "float", [n], b, sf.direction.forward, layout=lay)
+    assert p.launches() == 1 and p.describe()["layout"]["direct"] == 1
+    a = torch.from_numpy(x).cuda()
+    ref = np.fft.fft(x[at_in].astype(np.complex128))
+    for part in (b, max(1, b - 2)):
+        o = torch.full((int(at_out.max()) + 1,), 3 - 5j, dtype=a.dtype, device="cuda")
+        err = ctypes.create_string_buffer(_provider.ERR_CAP)
+        rc = p._lib.syclfft_b200_execute_batch(p._handle, a.data_ptr(), o.data_ptr(), part,
+                                               torch.cuda.current_stream().cuda_stream, err, _provider.ERR_CAP)
+        assert rc == 0, err.value
+        got = o.cpu().numpy()
+        assert rel_l2(got[at_out[:part]], ref[:part]) <= tol(n, dbl)
+        rest = np.ones(got.size, bool)
+        rest[at_out[:part].reshape(-1)] = False
+        assert np.all(got[rest] == np.complex64(3 - 5j))

@@ -8,7 +8,7 @@ import numpy as np
 import pytest
 
 from conftest import fp64_fft, gaussian_complex, norm_scale, rel_l2
-from native_libs import butterfly, describe, smooth_run
+from native_libs import butterfly, describe, smooth_run, smooth_run_line
 
 KK, CC, CK, KC = 0, 1, 2, 3
 
@@ -62,6 +62,33 @@ def test_fewer_lines_per_block(w_lines):
     x = gaussian_complex(100 * 7, 3, np.complex128)
     y = smooth_run(x, [100], 7, -1, w_lines=w_lines)
     assert rel_l2(y, fp64_fft(x, [100], 7, -1)) < 1e-13
+
+
+STRIDED = [
+    # (length, lines, in (line stride, element stride), out)
+    (64, 24, (1, 24), (64, 1)), (64, 24, (64, 1), (1, 24)), (60, 7, (1, 9), (1, 11)), (100, 5, (107, 1), (103, 1)),
+    (2048, 3, (1, 3), (2050, 1)), (1000, 17, (1001, 1), (1, 17)), (16, 1, (1, 3), (16, 1)), (24, 33, (1, 2), (24, 1)),
+    (1500, 9, (1, 9), (1500, 1)),
+]
+
+
+@pytest.mark.parametrize("double", [False, True])
+@pytest.mark.parametrize("n,b,src,dst", STRIDED, ids=str)
+def test_strided_lines_by_thread(n, b, src, dst, double):
+    """Strided one-dimensional plans against the transform of the gathered lines: contiguous or padded
+    lines, adjacent columns (of any pitch, overlapping reads included) on either side, partial tiles; no
+    element outside the output layout is written."""
+    at_in = np.arange(b)[:, None] * src[0] + np.arange(n)[None, :] * src[1]
+    at_out = np.arange(b)[:, None] * dst[0] + np.arange(n)[None, :] * dst[1]
+    x = gaussian_complex(int(at_in.max()) + 1, n + b, np.complex128)
+    out = np.full(int(at_out.max()) + 1, 7 - 3j)
+    for d, norm in ((-1, 1), (1, 0)):
+        y = smooth_run_line(x, n, b, src + dst, out, d, norm, double)
+        ref = (np.fft.fft(x[at_in]) if d < 0 else np.fft.ifft(x[at_in]) * n) * norm_scale(norm, d, n)
+        assert rel_l2(y[at_out], ref) < 1e-13
+        rest = np.ones(out.size, bool)
+        rest[at_out.reshape(-1)] = False
+        assert np.all(y[rest] == 7 - 3j)
 
 
 def test_dispatch():
