@@ -338,4 +338,40 @@ template <int R, class T, class C> SFB_HD void dft(C* v) {
     }
 }
 
+// Real transforms of length 2N over a complex FFT Z of length N.
+// X[k] = 1/2 [(Z[k] + conj Z[N-k]) - i W_2N^k (Z[k] - conj Z[N-k])] * scale; a = Z[k], c = Z[N-k]
+template <class C, class T> SFB_HD C real_post_pair(C a, C c, C w, T half) {
+    const C e = cmake<C>(a.x + c.x, a.y - c.y);
+    const C d = cmake<C>(a.x - c.x, a.y + c.y);
+    const T p = w.x * d.x - w.y * d.y, q = w.x * d.y + w.y * d.x;  // w * D
+    return cmake<C>((e.x + q) * half, (e.y - p) * half);
+}
+
+// Z[k] = (X[k] + conj X[N-k]) + i conj(W_2N^k) (X[k] - conj X[N-k]); a = X[k], c = X[N-k]
+template <class C, class T = decltype(C::x)> SFB_HD C real_pre_pair(C a, C c, C w) {
+    const C e = cmake<C>(a.x + c.x, a.y - c.y);
+    const C d = cmake<C>(a.x - c.x, a.y + c.y);
+    const T p = w.x * d.x + w.y * d.y, q = w.x * d.y - w.y * d.x;  // conj(w) * D
+    return cmake<C>(e.x - q, e.y + p);
+}
+
+// Both bins of a pair: a = Z[k], c = Z[N-k] become X[k], X[N-k] (w = W_2N^k; W_2N^(N-k) = -conj w, so the
+// second bin is made of the same sum, difference and product).
+template <class C, class T> SFB_HD void real_post_both(C& a, C& c, C w, T half) {
+    const C e = cmake<C>((a.x + c.x) * half, (a.y - c.y) * half);
+    const C d = cmake<C>((a.x - c.x) * half, (a.y + c.y) * half);
+    const C p = cmul(w, d);
+    a = cmake<C>(e.x + p.y, e.y - p.x);
+    c = cmake<C>(e.x - p.y, -e.y - p.x);
+}
+
+// The reverse: a = X[k], c = X[N-k] become Z[k], Z[N-k].
+template <class C> SFB_HD void real_pre_both(C& a, C& c, C w) {
+    const C e = cmake<C>(a.x + c.x, a.y - c.y);
+    const C d = cmake<C>(a.x - c.x, a.y + c.y);
+    const C q = cmul(cconj(w), d);
+    a = cmake<C>(e.x - q.y, e.y + q.x);
+    c = cmake<C>(e.x + q.y, q.x - e.y);
+}
+
 }  // namespace sfb

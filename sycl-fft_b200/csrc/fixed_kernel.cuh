@@ -119,24 +119,6 @@ __device__ __forceinline__ C fixed_load(const C* p) {
     else return *p;
 }
 
-// X[k] = 1/2 [(Z[k] + conj Z[N-k]) - i W_2N^k (Z[k] - conj Z[N-k])] * scale; a = Z[k], c = Z[N-k]
-template <class C, class T>
-__device__ __forceinline__ C real_post_pair(C a, C c, C w, T half) {
-    const C e = cmake<C>(a.x + c.x, a.y - c.y);
-    const C d = cmake<C>(a.x - c.x, a.y + c.y);
-    const T p = w.x * d.x - w.y * d.y, q = w.x * d.y + w.y * d.x;  // w * D
-    return cmake<C>((e.x + q) * half, (e.y - p) * half);
-}
-
-// Z[k] = (X[k] + conj X[N-k]) + i conj(W_2N^k) (X[k] - conj X[N-k]); a = X[k], c = X[N-k]
-template <class C, class T = decltype(C::x)>
-__device__ __forceinline__ C real_pre_pair(C a, C c, C w) {
-    const C e = cmake<C>(a.x + c.x, a.y - c.y);
-    const C d = cmake<C>(a.x - c.x, a.y + c.y);
-    const T p = w.x * d.x + w.y * d.y, q = w.x * d.y - w.y * d.x;  // conj(w) * D
-    return cmake<C>(e.x - q, e.y + p);
-}
-
 template <class T>
 struct FixedCtx {
     using C = cplx<T>;

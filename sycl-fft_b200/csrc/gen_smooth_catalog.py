@@ -11,7 +11,8 @@ cycles per line: issue slots of the butterflies, twiddles and addresses, shared-
 a bank simulation of every exchange, and the bytes in flight of the blocks that fit an SM. The model's
 first choices are within 10% of the fastest on average and up to 2x off for single lengths, so the
 committed catalog holds the fastest of 20,000 candidates timed on B200 (128 MB of input each). A
-length is left out where the power-of-two kernel of fixed_catalog.h was faster (64-point float lines).
+complex length is left out where the power-of-two kernel of fixed_catalog.h was faster (64-point float
+lines). The real transforms (FEAT 2 and 4) take the layouts chosen for complex lines.
 """
 import itertools
 import math
@@ -240,7 +241,8 @@ def best(dbl, kind, n, keep=KEEP):
     return [lay for _, lay in sorted(result.values(), key=lambda v: v[0])[:keep]]
 
 
-# (mapping, four-step twiddle, longest float line, longest double line)
+# (mapping, feature, longest float line, longest double line); the real transforms of feature 2 and 4 take
+# the layout chosen for the complex lines of half their length
 FAMILIES = (
     (KK, 0, 16384, 8192),
     (CC, 0, 2048, 2048),
@@ -255,9 +257,9 @@ def work(job):
     return job, best(dbl, kind, n)
 
 
-def entry(l, tw4):
+def entry(l, feat):
     return "%d, %d, %d, %d, %d, %d, %d, %d, %d, %d, %s" % (
-        l.dbl, l.kind, tw4, l.n, l.tpl, l.w, l.pads, l.pitch, l.threads, l.minb(), ", ".join(map(str, l.rs)))
+        l.dbl, l.kind, feat, l.n, l.tpl, l.w, l.pads, l.pitch, l.threads, l.minb(), ", ".join(map(str, l.rs)))
 
 
 def candidates():
@@ -282,9 +284,9 @@ def candidates():
 HEAD = """// Written by gen_smooth_catalog.py: the size-specialised kernels of the 7-smooth lengths
 // (smooth_kernel.cuh).
 //
-// X(ID, DOUBLE, KIND, TW4, N, TPL, W, PADS, PITCH, MAXT, MINB, RADICES...)
+// X(ID, DOUBLE, KIND, FEAT, N, TPL, W, PADS, PITCH, MAXT, MINB, RADICES...)
 //   KIND: 0 whole contiguous lines, 1 strided columns, 2 columns stored as rows, 3 rows stored as
-//   columns; TW4: four-step twiddle on the store; TPL threads per line; W lines per CTA (KIND 0:
+//   columns; FEAT: 1 four-step twiddle on the store, 2 / 4 R2C / C2R of twice the length; TPL threads per line; W lines per CTA (KIND 0:
 //   at most); shared-memory rows of PITCH elements, one padding element per 2^PADS (0: none);
 //   RADICES the Stockham stages in order.
 // SFB_SMOOTH_PART_<p> lists the entries that smooth_variants.cu compiles as part p.

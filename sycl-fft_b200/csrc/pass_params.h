@@ -31,6 +31,9 @@ enum : int { kModeK = 0, kModeC = 1 };         // thread mapping / coalesced dim
 // Thread mappings of smooth_kernel.cuh, input side then output side: K lanes walk a line's elements
 // (element stride 1), C lanes walk adjacent lines (line stride 1).
 enum : int { kSmoothKK = 0, kSmoothCC = 1, kSmoothCK = 2, kSmoothKC = 3 };
+// Features of a smooth_kernel.cuh instantiation: four-step twiddle on the store; real transforms of length
+// 2N, bins formed after the last stage (R2C) or read before the first (C2R).
+enum : int { kSmoothTw4 = 1, kSmoothPost = 2, kSmoothPre = 4 };
 // Rows of a radix-R stage's twiddle table in smooth_kernel.cuh: W^(r*jm) for r = 1, 2, 4, 8 below R.
 #if defined(__CUDACC__)
 __host__ __device__

@@ -404,27 +404,13 @@ struct Builder {
         use_base_table(ps);
     }
 
-    // Stage twiddles of a smooth_catalog.h kernel: per stage the rows W_(ns*R)^(r*jm), jm < ns, for
-    // r = 1, 2, 4, 8 below R.
+    // Stage twiddles of a smooth_catalog.h kernel.
     int smooth_table(const SmoothEntry& e) {
         std::vector<int> key(e.radices, e.radices + e.nstages);
         key.push_back(-2);  // distinct from the other table layouts of the radices
         auto it = seq_tables.find(key);
         if (it != seq_tables.end()) return it->second;
-        std::vector<int64_t> ckey(e.radices, e.radices + e.nstages);
-        ckey.push_back(-600);
-        auto tw = cached_table(ckey, [&] {
-            std::vector<std::complex<double>> t;
-            int64_t ns = 1;
-            for (int s = 0; s < e.nstages; ++s) {
-                const int R = e.radices[s];
-                for (int q = 0; q < smooth_tw_entries(R); ++q)
-                    for (int64_t jm = 0; jm < ns; ++jm) t.push_back(cis_neg((int64_t(1) << q) * jm, ns * R));
-                ns *= R;
-            }
-            return t;
-        });
-        const int id = add_table(*tw);
+        const int id = add_table(smooth_twiddles(e));
         seq_tables[key] = id;
         return id;
     }
@@ -457,7 +443,7 @@ struct Builder {
                 kind = kSmoothKK;
             }
         }
-        const SmoothEntry* e = find_smooth(req.dbl, kind, tw4, p.n);
+        const SmoothEntry* e = find_smooth(req.dbl, kind, tw4 ? kSmoothTw4 : 0, p.n);
         if (!e || static_cast<int64_t>(e->w) * e->pitch * cs > smem_limit) return;
         ps.tables.smooth = smooth_table(*e);
         ps.smooth_id = e->id;
@@ -1337,7 +1323,7 @@ struct Builder {
     void line_pass(Buf& cur) {
         const int64_t n = static_cast<int64_t>(req.shape[0]);
         const int kind = strided_line_kind(req.line_in, req.line_out);
-        const SmoothEntry* e = kind < 0 || n > (1 << 20) ? nullptr : find_smooth(req.dbl, kind, false, static_cast<int>(n));
+        const SmoothEntry* e = kind < 0 || n > (1 << 20) ? nullptr : find_smooth(req.dbl, kind, 0, static_cast<int>(n));
         if (!e || static_cast<int64_t>(e->w) * e->pitch * cs > smem_limit)
             throw std::runtime_error("no single-pass kernel for this strided length");
         PassSpec ps;
@@ -1644,8 +1630,8 @@ const FixedEntry* find_fixed(bool dbl, int mode, int n, int feat) {
 namespace {
 const std::vector<SmoothEntry>& smooth_entries() {
     static const std::vector<SmoothEntry> all = {
-#define SFB_X(ID, DBL, KIND, TW4, N, TPL, W, PADS, PITCH, MAXT, MINB, ...) \
-    {ID, DBL, KIND, TW4, N, TPL, W, PADS, PITCH, MAXT, MINB, {__VA_ARGS__}, count_args(__VA_ARGS__)},
+#define SFB_X(ID, DBL, KIND, FEAT, N, TPL, W, PADS, PITCH, MAXT, MINB, ...) \
+    {ID, DBL, KIND, FEAT, N, TPL, W, PADS, PITCH, MAXT, MINB, {__VA_ARGS__}, count_args(__VA_ARGS__)},
         SFB_SMOOTH_CATALOG(SFB_X)
 #undef SFB_X
     };
@@ -1653,14 +1639,30 @@ const std::vector<SmoothEntry>& smooth_entries() {
 }
 }  // namespace
 
-const SmoothEntry* find_smooth(bool dbl, int kind, bool tw4, int n) {
+const SmoothEntry* find_smooth(bool dbl, int kind, int feat, int n) {
     static const std::map<std::array<int, 4>, const SmoothEntry*> index = [] {
         std::map<std::array<int, 4>, const SmoothEntry*> m;
-        for (const SmoothEntry& e : smooth_entries()) m[{e.dbl, e.kind, e.tw4, e.n}] = &e;
+        for (const SmoothEntry& e : smooth_entries()) m[{e.dbl, e.kind, e.feat, e.n}] = &e;
         return m;
     }();
-    const auto it = index.find({dbl ? 1 : 0, kind, tw4 ? 1 : 0, n});
+    const auto it = index.find({dbl ? 1 : 0, kind, feat, n});
     return it == index.end() ? nullptr : it->second;
+}
+
+std::vector<std::complex<double>> smooth_twiddles(const SmoothEntry& e) {
+    std::vector<int64_t> key(e.radices, e.radices + e.nstages);
+    key.push_back(-600);
+    return *cached_table(key, [&] {
+        std::vector<std::complex<double>> t;
+        int64_t ns = 1;
+        for (int s = 0; s < e.nstages; ++s) {
+            const int R = e.radices[s];
+            for (int q = 0; q < smooth_tw_entries(R); ++q)
+                for (int64_t jm = 0; jm < ns; ++jm) t.push_back(cis_neg((int64_t(1) << q) * jm, ns * R));
+            ns *= R;
+        }
+        return t;
+    });
 }
 
 int strided_line_kind(const LineLayout& in, const LineLayout& out) {

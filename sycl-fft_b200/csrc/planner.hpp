@@ -116,11 +116,13 @@ bool has_fused4(bool dbl, int col_id, int row_id);
 // One entry of smooth_catalog.h as seen by the host. kind: kSmoothKK / CC / CK / KC, the lane mappings of the
 // input and output sides (smooth_kernel.cuh).
 struct SmoothEntry {
-    int id, dbl, kind, tw4, n, tpl, w, pads, pitch, maxt, minb;
+    int id, dbl, kind, feat, n, tpl, w, pads, pitch, maxt, minb;  // feat: kSmoothTw4 / Post / Pre
     int radices[kMaxStages];
     int nstages;
 };
-const SmoothEntry* find_smooth(bool dbl, int kind, bool tw4, int n);
+const SmoothEntry* find_smooth(bool dbl, int kind, int feat, int n);
+// Its stage twiddles: per stage the rows W_(ns*R)^(r*jm), jm < ns, for r = 1, 2, 4, 8 below R.
+std::vector<std::complex<double>> smooth_twiddles(const SmoothEntry& e);
 const SmoothEntry* smooth_entry(int id);
 // The mapping pair of a strided one-dimensional layout, or -1 when a side is neither contiguous lines nor
 // adjacent columns.

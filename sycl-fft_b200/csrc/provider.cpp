@@ -256,9 +256,10 @@ struct DevicePlan {
     int64_t real_n = 0;             // real length N (even)
     std::unique_ptr<DevicePlan> inner;
     void* real_buf = nullptr;       // half-length spectra: batch x N/2 complex
-    void* real_tw = nullptr;        // W_N^k, k = 0..N/2 (then the fused kernel's base twiddles)
+    void* real_tw = nullptr;        // W_N^k, k = 0..N/2 (then the one-pass kernel's stage twiddles)
     const RealFusedEntry* real_fused = nullptr;  // one-pass kernel for N/2 (real_kernel.cu), or none
-    int64_t real_base_off = 0;      // complex elements from real_tw to the base twiddles
+    const SmoothEntry* real_smooth = nullptr;    // or the one-pass smooth_catalog.h kernel
+    int64_t real_base_off = 0;      // complex elements from real_tw to the stage twiddles
     // Real transforms of rank 2-3: `inner` is the 1D real plan of the last axis over every outer
     // line, `outer` the complex plan over the outer axes (last axis untransformed), md_buf the
     // C2R intermediate (batch x outer lines x (N/2+1) complex).
@@ -756,13 +757,23 @@ DevicePlan* create_real_plan_1d(const syclfft_b200_plan_config_v1& cfg, int kind
     const bool dbl = plan->spec.req.dbl;
     const size_t cs = dbl ? 16 : 8;
     const uint64_t h = n / 2;
-    // One pass when N/2 has a fused kernel (not for split-precision plans, whose inner FFT runs
-    // on the tensor cores); SYCLFFT_B200_REAL_FUSED=0 keeps the two-pass form.
+    // One pass when N/2 has a smooth_catalog.h kernel with the pre- / post-process (every 7-smooth N/2 that
+    // fits a block; not for split-precision plans, whose inner FFT runs on the tensor cores):
+    // 1.03x to 1.4x the power-of-two kernels of real_kernel.cu and 2.1x (geometric mean over 286 lengths) the
+    // two-pass form. SYCLFFT_B200_REAL_FUSED=0 keeps the two-pass form, =fixed the kernels of real_kernel.cu.
     const char* fused_env = std::getenv("SYCLFFT_B200_REAL_FUSED");
+    const char* generic = std::getenv("SYCLFFT_B200_KERNELS");
     const bool split = !dbl && (flags & SYCLFFT_B200_CREATE_SPLIT_BF16) != 0;
-    if (!split && !(fused_env && std::strcmp(fused_env, "0") == 0))
-        plan->real_fused = find_real_fused(dbl, static_cast<int64_t>(h));
-    plan->spec.scratch_elements = plan->real_fused ? 0 : inner->spec.scratch_elements + h * cfg.batch_count;
+    if (!split && !(fused_env && std::strcmp(fused_env, "0") == 0)) {
+        const bool take = !(fused_env && std::strcmp(fused_env, "fixed") == 0) &&
+                          !(generic && std::strcmp(generic, "generic") == 0) && h <= (1u << 20);
+        if (take)
+            plan->real_smooth = find_smooth(dbl, kSmoothKK, kind == SYCLFFT_B200_REAL_R2C ? kSmoothPost : kSmoothPre,
+                                            static_cast<int>(h));
+        if (!plan->real_smooth) plan->real_fused = find_real_fused(dbl, static_cast<int64_t>(h));
+    }
+    const bool one_pass = plan->real_fused || plan->real_smooth;
+    plan->spec.scratch_elements = one_pass ? 0 : inner->spec.scratch_elements + h * cfg.batch_count;
     DeviceGuard guard(plan->device);
     cudaStream_t ms = memory_stream(plan->device);
     std::vector<std::complex<double>> table;
@@ -775,6 +786,9 @@ DevicePlan* create_real_plan_1d(const syclfft_b200_plan_config_v1& cfg, int kind
             for (int64_t jm = 0; jm < ns; ++jm) table.push_back(cis_neg(jm, ns * R));
             ns *= R;
         }
+    } else if (plan->real_smooth) {
+        const auto t = smooth_twiddles(*plan->real_smooth);
+        table.insert(table.end(), t.begin(), t.end());
     }
     std::vector<unsigned char> tw(table.size() * cs);
     for (size_t k = 0; k < table.size(); ++k) {
@@ -788,7 +802,7 @@ DevicePlan* create_real_plan_1d(const syclfft_b200_plan_config_v1& cfg, int kind
     }
     check(cudaMallocAsync(&plan->real_tw, tw.size(), ms), "cudaMallocAsync(real twiddles)");
     check(cudaMemcpyAsync(plan->real_tw, tw.data(), tw.size(), cudaMemcpyHostToDevice, ms), "cudaMemcpy(real twiddles)");
-    if (!plan->real_fused)
+    if (!one_pass)
         check(cudaMallocAsync(&plan->real_buf, h * cfg.batch_count * cs, ms), "cudaMallocAsync(real spectra)");
     check(cudaStreamSynchronize(ms), "real plan tables");
     check(cudaEventCreateWithFlags(&plan->done, cudaEventDisableTiming), "cudaEventCreate");
@@ -990,7 +1004,7 @@ DevicePlan* create_strided_plan(const syclfft_b200_plan_config_v1& cfg, const sy
         const char* generic = std::getenv("SYCLFFT_B200_KERNELS");
         const int kind = strided_line_kind(li, lo);
         if (kind >= 0 && !split && !(generic && std::strcmp(generic, "generic") == 0) && cfg.lengths[0] <= (1u << 20) &&
-            find_smooth(dbl, kind, false, static_cast<int>(cfg.lengths[0]))) {
+            find_smooth(dbl, kind, 0, static_cast<int>(cfg.lengths[0]))) {
             std::unique_ptr<DevicePlan> inner(create_plan(cfg, flags | SYCLFFT_B200_CREATE_SYNC, 0, &li, &lo));
             auto plan = std::make_unique<DevicePlan>();
             plan->device = inner->device;
@@ -1120,6 +1134,17 @@ void execute_real(DevicePlan* plan, const void* in, void* out, cudaStream_t stre
         check(launch_real_fused(*plan->real_fused, plan->real_kind == SYCLFFT_B200_REAL_R2C, in, out, lines,
                                 plan->real_tw, base, scale, stream),
               "fused real transform");
+    } else if (plan->real_smooth) {
+        const bool r2c = plan->real_kind == SYCLFFT_B200_REAL_R2C;
+        SmoothParams p;
+        p.n_cols = lines;
+        p.in_cs = r2c ? h : h + 1;
+        p.out_cs = r2c ? h + 1 : h;
+        p.tw = static_cast<const unsigned char*>(plan->real_tw) + plan->real_base_off * (dbl ? 16 : 8);
+        p.real_tw = plan->real_tw;
+        p.conj_in = p.conj_out = r2c ? 0 : 1;  // C2R: the unnormalized inverse as conj(FFT(conj z))
+        p.scale = scale;
+        check(launch_smooth(*plan->real_smooth, p, 1, plan->sms, in, out, stream), "fused real transform");
     } else if (plan->real_kind == SYCLFFT_B200_REAL_R2C) {
         execute_plan(plan->inner.get(), in, plan->real_buf, stream, batch, 0, -1);
         check(launch_r2c_post(dbl, plan->real_buf, out, h, lines, plan->real_tw, scale, stream), "R2C post-process");
@@ -1784,12 +1809,12 @@ SYCLFFT_B200_EXPORT int syclfft_b200_describe_plan(const void* plan, char* buf, 
         const sfb::DevicePlan* last = p->inner.get();
         s = std::string("{\"real\":\"") + (p->real_kind == SYCLFFT_B200_REAL_R2C ? "r2c" : "c2r") +
             "\",\"n\":" + std::to_string(p->real_n) + ",\"shape\":[" + shape + "],\"fused\":" +
-            (last->real_fused ? "1" : "0") + ",\"inner\":" + sfb::describe_plan(last->inner->spec) +
+            (last->real_fused || last->real_smooth ? "1" : "0") + ",\"inner\":" + sfb::describe_plan(last->inner->spec) +
             ",\"outer\":" + sfb::describe_plan(p->outer->spec) + "}";
     } else if (p->real_kind) {
         // a real plan: its complex plan of half the length and the pre-/post-process pass
         s = std::string("{\"real\":\"") + (p->real_kind == SYCLFFT_B200_REAL_R2C ? "r2c" : "c2r") +
-            "\",\"n\":" + std::to_string(p->real_n) + ",\"fused\":" + (p->real_fused ? "1" : "0") +
+            "\",\"n\":" + std::to_string(p->real_n) + ",\"fused\":" + (p->real_fused || p->real_smooth ? "1" : "0") +
             ",\"inner\":" + sfb::describe_plan(p->inner->spec) + "}";
     } else if (p->strided) {
         auto side = [](const sfb::Layout& l, bool contig) {
@@ -1832,9 +1857,9 @@ SYCLFFT_B200_EXPORT int syclfft_b200_plan_launches(const void* plan) {
     if (!p) return -1;
     if (p->real_md) {
         const sfb::DevicePlan* last = p->inner.get();
-        return (last->real_fused ? 1 : sfb::pass_launches(last->inner.get()) + 1) + sfb::pass_launches(p->outer.get());
+        return (last->real_fused || last->real_smooth ? 1 : sfb::pass_launches(last->inner.get()) + 1) + sfb::pass_launches(p->outer.get());
     }
-    if (p->real_kind) return p->real_fused ? 1 : sfb::pass_launches(p->inner.get()) + 1;
+    if (p->real_kind) return p->real_fused || p->real_smooth ? 1 : sfb::pass_launches(p->inner.get()) + 1;
     if (p->strided)
         return sfb::pass_launches(p->inner.get()) +
                (p->interleaved || p->direct ? 0 : (p->in_contig ? 0 : 1) + (p->out_contig ? 0 : 1));

@@ -10,9 +10,10 @@
 // Each thread handles the pair (k, H - k), so both of its values are read once; the
 // normalization scale is fused.
 //
-// Where the half length H has a size-specialised single-CTA kernel (the catalog below), the
-// pre-/post-process is fused into it instead (kFeatRealPre / kFeatRealPost of
-// fixed_kernel.cuh): one HBM pass per real transform.
+// These two are for the lengths without a one-pass kernel (half lengths with a factor above 7, or longer
+// than a block holds); 7-smooth half lengths run on smooth_kernel.cuh with the process fused into the
+// transform. The power-of-two kernels below (kFeatRealPre / kFeatRealPost of fixed_kernel.cuh) do the
+// same; they are taken under SYCLFFT_B200_REAL_FUSED=fixed.
 #include <atomic>
 #include <type_traits>
 

@@ -43,6 +43,7 @@ struct SmoothParams {
     const void* tw4_hi = nullptr;
     const void* tw4_lo = nullptr;
     int tw4_shift = 0, tw4_conj = 0;
+    const void* real_tw = nullptr;  // W_2N^k, k = 0..N (real transforms of length 2N)
 };
 
 // Twiddles of one butterfly, u[r] *= w^r with w = W_(Ns*R)^jm. The table holds w, w^2, w^4 and w^8 for every
@@ -107,6 +108,7 @@ struct SmoothCtx {
     const C *tw4_hi, *tw4_lo;
     int tw4_shift;
     T tw4_sy;
+    const C* real_tw;
 };
 
 // Four-step twiddles of one butterfly's outputs k = j + r * NR of column c: W^(k*c) = W^(j*c) * s^r with
@@ -141,7 +143,7 @@ __device__ __forceinline__ void smooth_tw4(C* u, const SmoothCtx<T>& X, int j) {
 
 // KIND: the mapping pair; a stage's reads and writes use the mapping of its phase. Shared memory
 // holds one row of PITCH elements per line, one padding element per 2^PADS (0: none).
-template <class T, int N, int TPL, int KIND, int W, int PADS, int PITCH, bool TW4, int NS, int TWOFF, int R, bool FIRST,
+template <class T, int N, int TPL, int KIND, int W, int PADS, int PITCH, int FEAT, int NS, int TWOFF, int R, bool FIRST,
           bool LAST>
 __device__ __forceinline__ void smooth_stage(SmoothCtx<T>& X) {
     using C = cplx<T>;
@@ -162,7 +164,8 @@ __device__ __forceinline__ void smooth_stage(SmoothCtx<T>& X) {
     for (int i = 0; i < NB; ++i) {
         const int j = t + i * TPL;
         if (act && (EXACT || i + 1 < NB || j < NR)) {
-            if constexpr (FIRST) {
+            if constexpr (FIRST && !(FEAT & kSmoothPre)) {
+
                 if (X.in_ok) {
                     const C* g = CMAP ? X.gin + (int64_t)j * X.in_ks : X.gin + j;
 #pragma unroll
@@ -185,7 +188,7 @@ __device__ __forceinline__ void smooth_stage(SmoothCtx<T>& X) {
             }
         }
     }
-    if constexpr (!FIRST && !LAST) __syncthreads();
+    if constexpr ((!FIRST || (FEAT & kSmoothPre)) && !LAST) __syncthreads();
 #pragma unroll
     for (int i = 0; i < NB; ++i) {
         const int j = t + i * TPL;
@@ -194,9 +197,13 @@ __device__ __forceinline__ void smooth_stage(SmoothCtx<T>& X) {
             const int jm = LAST ? j : j % NS;
             if constexpr (NS > 1) smooth_twiddle<R, NS>(u, X.tw + TWOFF, jm);
             dft<R, T>(u);
-            if constexpr (LAST) {
+            if constexpr (LAST && (FEAT & kSmoothPost)) {
+                // over the elements this thread read; the bins are formed from pairs after a barrier
+#pragma unroll
+                for (int r = 0; r < R; ++r) row[smooth_idx<PADS>(j + r * NR)] = u[r];
+            } else if constexpr (LAST) {
                 if (X.out_ok) {
-                    if constexpr (TW4) smooth_tw4<R, NR>(u, X, j);
+                    if constexpr (FEAT & kSmoothTw4) smooth_tw4<R, NR>(u, X, j);
                     C* g = CMAP ? X.gout + (int64_t)j * X.out_ks : X.gout + j;
 #pragma unroll
                     for (int r = 0; r < R; ++r) {
@@ -223,22 +230,92 @@ __device__ __forceinline__ void smooth_stage(SmoothCtx<T>& X) {
     if constexpr (!LAST) __syncthreads();
 }
 
-template <class T, int N, int TPL, int KIND, int W, int PADS, int PITCH, bool TW4, int NS, int TWOFF, bool FIRST, int R,
+template <class T, int N, int TPL, int KIND, int W, int PADS, int PITCH, int FEAT, int NS, int TWOFF, bool FIRST, int R,
           int... Rest>
 __device__ __forceinline__ void smooth_stages(SmoothCtx<T>& X) {
     constexpr bool LAST = sizeof...(Rest) == 0;
-    smooth_stage<T, N, TPL, KIND, W, PADS, PITCH, TW4, NS, TWOFF, R, FIRST, LAST>(X);
+    smooth_stage<T, N, TPL, KIND, W, PADS, PITCH, FEAT, NS, TWOFF, R, FIRST, LAST>(X);
     if constexpr (!LAST)
-        smooth_stages<T, N, TPL, KIND, W, PADS, PITCH, TW4, NS * R, TWOFF + NS * smooth_tw_entries(R), false, Rest...>(
+        smooth_stages<T, N, TPL, KIND, W, PADS, PITCH, FEAT, NS * R, TWOFF + NS * smooth_tw_entries(R), false, Rest...>(
             X);
+}
+
+// Real transforms: bins k and N - k of each line from its spectrum in shared memory, and the reverse. One
+// thread takes the pair, so each value moves once and the two bins share their arithmetic; the loads of a
+// group of pairs are issued before the first is used.
+template <class T, int N, int TPL, int PADS, int PITCH>
+__device__ __forceinline__ void smooth_post(SmoothCtx<T>& X) {
+    using C = cplx<T>;
+    constexpr int NP = N / 2 + 1, G = 4;
+    __syncthreads();
+    if (!X.out_ok) return;
+    const T half = T(0.5) * X.sx;
+    const C* row = X.sm + X.w_out * PITCH;
+    for (int k0 = X.t_out; k0 < NP; k0 += G * TPL) {
+        C a[G], c[G], w[G];
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+            const int k = k0 + g * TPL, kk = N - k;
+            if (k < NP) {
+                w[g] = __ldg(X.real_tw + k);
+                a[g] = row[smooth_idx<PADS>(k)];
+                c[g] = row[smooth_idx<PADS>(k == 0 ? 0 : kk)];
+            }
+        }
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+            const int k = k0 + g * TPL, kk = N - k;
+            if (k < NP) {
+                real_post_both(a[g], c[g], w[g], half);
+                X.gout[k] = a[g];
+                if (kk != k) X.gout[kk] = c[g];
+            }
+        }
+    }
+}
+
+template <class T, int N, int TPL, int PADS, int PITCH>
+__device__ __forceinline__ void smooth_pre(SmoothCtx<T>& X) {
+    using C = cplx<T>;
+    constexpr int NP = N / 2 + 1, G = sizeof(T) == 4 ? 6 : 4;
+    C* row = X.sm + X.w_in * PITCH;
+    if (X.act_in) {
+        for (int k0 = X.t_in; k0 < NP; k0 += G * TPL) {
+            C a[G], c[G], w[G];
+#pragma unroll
+            for (int g = 0; g < G; ++g) {
+                const int k = k0 + g * TPL;
+                a[g] = c[g] = w[g] = cmake<C>(T(0), T(0));
+                if (k < NP && X.in_ok) {
+                    a[g] = X.gin[k];
+                    c[g] = X.gin[N - k];
+                    w[g] = __ldg(X.real_tw + k);
+                }
+            }
+#pragma unroll
+            for (int g = 0; g < G; ++g) {
+                const int k = k0 + g * TPL, kk = N - k;
+                if (k < NP) {
+                    if (k == 0) a[g].y = c[g].y = T(0);  // bins 0 and N of a real signal are real
+                    real_pre_both(a[g], c[g], w[g]);
+                    a[g].y *= X.in_sy;
+                    c[g].y *= X.in_sy;
+                    row[smooth_idx<PADS>(k)] = a[g];
+                    if (kk != k && k > 0) row[smooth_idx<PADS>(kk)] = c[g];
+                }
+            }
+        }
+    }
+    __syncthreads();
 }
 
 // grid = n_outer * col_tiles; KK: block >= w * TPL, other mappings: block = round_up(W * TPL, 32);
 // dynamic smem: lines * PITCH complex values.
-template <class T, int N, int TPL, int KIND, int W, int PADS, int PITCH, bool TW4, int MAXT, int MINB, int... Rs>
+template <class T, int N, int TPL, int KIND, int W, int PADS, int PITCH, int FEAT, int MAXT, int MINB, int... Rs>
 __global__ void __launch_bounds__(MAXT, MINB)
     fft_smooth_kernel(const __grid_constant__ SmoothParams P, const cplx<T>* in, cplx<T>* out) {
     using C = cplx<T>;
+    static_assert(!(FEAT & (kSmoothPost | kSmoothPre)) || KIND == kSmoothKK, "whole contiguous lines");
     extern __shared__ __align__(16) unsigned char smem_raw[];
     SmoothCtx<T> X;
     X.sm = reinterpret_cast<C*>(smem_raw);
@@ -250,6 +327,7 @@ __global__ void __launch_bounds__(MAXT, MINB)
     X.sy = P.conj_out ? -X.sx : X.sx;
     X.in_ks = P.in_ks;
     X.out_ks = P.out_ks;
+    X.real_tw = static_cast<const C*>(P.real_tw);
     const int tid = threadIdx.x;
     constexpr bool CIN = KIND == kSmoothCC || KIND == kSmoothCK, COUT = KIND == kSmoothCC || KIND == kSmoothKC;
     const int lines = KIND == kSmoothKK ? P.w : W;
@@ -268,14 +346,16 @@ __global__ void __launch_bounds__(MAXT, MINB)
     X.out_ok = X.act_out && co < P.n_cols;
     X.gin = in + o * P.in_hi + (CIN ? ci : ci * P.in_cs);
     X.gout = out + o * P.out_hi + (COUT ? co : co * P.out_cs);
-    if constexpr (TW4) {
+    if constexpr (FEAT & kSmoothTw4) {
         X.sel = static_cast<int>(co);
         X.tw4_hi = static_cast<const C*>(P.tw4_hi);
         X.tw4_lo = static_cast<const C*>(P.tw4_lo);
         X.tw4_shift = P.tw4_shift;
         X.tw4_sy = (P.tw4_conj != P.conj_out) ? T(-1) : T(1);
     }
-    smooth_stages<T, N, TPL, KIND, W, PADS, PITCH, TW4, 1, 0, true, Rs...>(X);
+    if constexpr (FEAT & kSmoothPre) smooth_pre<T, N, TPL, PADS, PITCH>(X);
+    smooth_stages<T, N, TPL, KIND, W, PADS, PITCH, FEAT, 1, 0, true, Rs...>(X);
+    if constexpr (FEAT & kSmoothPost) smooth_post<T, N, TPL, PADS, PITCH>(X);
 }
 
 }  // namespace sfb

@@ -13,9 +13,9 @@ namespace sfb {
 
 const SmoothKernel* SFB_CAT(smooth_part_, SFB_SMOOTH_PART)(int* count) {
     static const SmoothKernel kernels[] = {
-#define SFB_X(ID, DBL, KIND, TW4, N, TPL, W, PADS, PITCH, MAXT, MINB, ...)                                       \
+#define SFB_X(ID, DBL, KIND, FEAT, N, TPL, W, PADS, PITCH, MAXT, MINB, ...)                                       \
     {ID, reinterpret_cast<const void*>(&fft_smooth_kernel<std::conditional_t<(DBL) != 0, double, float>, N, TPL, \
-                                                          KIND, W, PADS, PITCH, (TW4) != 0, MAXT, MINB, __VA_ARGS__>)},
+                                                          KIND, W, PADS, PITCH, FEAT, MAXT, MINB, __VA_ARGS__>)},
         SFB_CAT(SFB_SMOOTH_PART_, SFB_SMOOTH_PART)(SFB_X)
 #undef SFB_X
     };

@@ -70,3 +70,13 @@ extern "C" int sfb_check_powers_f64(int mode, int radix, double wr, double wi, c
 extern "C" int sfb_check_powers_f32(int mode, int radix, float wr, float wi, const float* in, float* out) {
     return powers_dispatch<float>(mode, radix, wr, wi, in, out);
 }
+
+// Both bins of a real-transform pair (real_post_both / real_pre_both), in and out: a, c, w as re, im.
+extern "C" void sfb_check_real_pair(int pre, double half, const double* in, double* out) {
+    using C = sfb::cplx<double>;
+    C a = sfb::cmake<C>(in[0], in[1]), c = sfb::cmake<C>(in[2], in[3]);
+    const C w = sfb::cmake<C>(in[4], in[5]);
+    if (pre) sfb::real_pre_both(a, c, w);
+    else sfb::real_post_both(a, c, w, half);
+    out[0] = a.x; out[1] = a.y; out[2] = c.x; out[3] = c.y;
+}

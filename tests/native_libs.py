@@ -136,3 +136,14 @@ def smooth_run_line(x, n, batch, layout, out, direction, norm=0, double=False, i
     if rc:
         raise RuntimeError(err.value.decode() or "no single-pass kernel")
     return got
+
+
+def real_pair(pre, a, c, w, half=0.5):
+    """The two bins of a real-transform pair through the kernels' pair functions."""
+    L = _load("libbutterfly_check.so")
+    L.sfb_check_real_pair.argtypes = [ctypes.c_int, ctypes.c_double, ctypes.c_void_p, ctypes.c_void_p]
+    L.sfb_check_real_pair.restype = None
+    xin = np.array([a.real, a.imag, c.real, c.imag, w.real, w.imag])
+    out = np.zeros(4)
+    L.sfb_check_real_pair(int(pre), float(half), xin.ctypes.data, out.ctypes.data)
+    return out[0] + 1j * out[1], out[2] + 1j * out[3]

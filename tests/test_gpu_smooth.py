@@ -76,3 +76,31 @@ def test_strided_lines(sf, torch, n, b, src, dst, dbl):
         rest = np.ones(got.size, bool)
         rest[at_out[:part].reshape(-1)] = False
         assert np.all(got[rest] == np.complex64(3 - 5j))
+
+
+@pytest.mark.parametrize("dbl", [False, True], ids=["float", "double"])
+@pytest.mark.parametrize("h,batch", [(16, 5), (45, 97), (64, 3), (105, 26), (1000, 3), (2187, 2), (4096, 2), (6125, 2), (8000, 2),
+                                     (13440, 2), (15625, 1)], ids=str)
+def test_real_one_pass(sf, torch, h, batch, dbl):
+    """Real transforms of length 2h in one launch, odd and even half lengths, against FP64 rfft / irfft; the
+    imaginary parts of bins 0 and h do not matter."""
+    n = 2 * h
+    rt, ct = (np.float64, np.complex128) if dbl else (np.float32, np.complex64)
+    rng = np.random.default_rng(n)
+    x = rng.uniform(-1, 1, (batch, n)).astype(rt)
+    fits = not dbl or h <= 8192
+    opts = sf.plan_options(normalization=sf.normalization.orthogonal)
+    f = sf.plan_dft_r2c_1d("double" if dbl else "float", n, batch, opts)
+    b = sf.plan_dft_c2r_1d("double" if dbl else "float", n, batch, opts)
+    if fits:
+        assert f.launches() == 1 and b.launches() == 1
+    spec = torch.full((batch * (h + 1),), 9.0, dtype=f.dtype, device="cuda")
+    f.execute(torch.from_numpy(x).cuda(), spec).synchronize()
+    ref = np.fft.rfft(x.astype(np.float64), axis=1, norm="ortho")
+    assert rel_l2(spec.cpu().numpy(), ref.reshape(-1)) <= tol(n, dbl)
+    s = ref.astype(ct)
+    s[:, 0] += 3j
+    s[:, h] -= 2j
+    back = torch.full((batch * n,), 9.0, dtype=b.real_dtype, device="cuda")
+    b.execute(torch.from_numpy(s).cuda(), back).synchronize()
+    assert rel_l2(back.cpu().numpy(), x.reshape(-1).astype(np.float64)) <= 2 * tol(n, dbl)

@@ -8,7 +8,7 @@ import numpy as np
 import pytest
 
 from conftest import fp64_fft, gaussian_complex, norm_scale, rel_l2
-from native_libs import butterfly, describe, smooth_run, smooth_run_line
+from native_libs import butterfly, describe, real_pair, smooth_run, smooth_run_line
 
 KK, CC, CK, KC = 0, 1, 2, 3
 
@@ -33,13 +33,13 @@ def test_catalog_geometry():
     assert [e[0] for e in entries] == list(range(len(entries)))
     assert len({(e[1], e[2], e[3], e[4]) for e in entries}) == len(entries)
     for e in entries:
-        _, dbl, kind, tw4, n, tpl, w, pads, pitch, maxt, minb, *radices = e
+        _, dbl, kind, feat, n, tpl, w, pads, pitch, maxt, minb, *radices = e
         assert np.prod(radices) == n and len(radices) >= 2 and max(radices) <= 16, e
         assert (w * tpl + 31) // 32 * 32 == maxt <= 1024 and maxt * minb <= 2048, e
         assert pitch > (n - 1) + ((n - 1) >> pads if pads else 0), e
         assert w * pitch * (16 if dbl else 8) <= 227 * 1024, e
         assert kind == KK or w & (w - 1) == 0, e
-        assert not tw4 or kind == CC, e
+        assert feat in (0, {KK: 0, CC: 1}.get(kind, 0)) or (kind == KK and feat in (2, 4)), e
 
 
 # the shortest and longest lines of each mapping, one with idle threads in a stage, several lines per block
@@ -102,3 +102,18 @@ def test_dispatch():
     assert ids([840, 1200]) == [True, True]
     assert ids([256, 256], split_bf16=True) == [False, False]
     assert ids([1009]) == [False]
+
+
+@pytest.mark.parametrize("n", [1, 6, 15])
+def test_real_pairs(n):
+    """Bins k and n - k of a real line of 2n points from its half-length spectrum, and back."""
+    rng = np.random.default_rng(n)
+    x = rng.standard_normal(2 * n)
+    z = np.fft.fft(x[0::2] + 1j * x[1::2])
+    ref = np.fft.rfft(x)
+    for k in range(n // 2 + 1):
+        w = np.exp(-1j * np.pi * k / n)
+        a, c = real_pair(False, z[k], z[(n - k) % n], w)
+        assert abs(a - ref[k]) < 1e-12 and abs(c - ref[n - k]) < 1e-12
+        p, q = real_pair(True, ref[k], ref[n - k], w)
+        assert abs(p - 2 * z[k]) < 1e-12 and (k == 0 or abs(q - 2 * z[n - k]) < 1e-12)
