@@ -7,11 +7,13 @@
 #include "smooth_catalog.h"
 #include "tc_catalog.h"
 #include "bluestein_catalog.h"
+#include "conv_catalog.h"
 #include "tc_shape.h"
 
 #include <algorithm>
 #include <array>
 #include <cmath>
+#include <initializer_list>
 #include <limits>
 #include <map>
 #include <memory>
@@ -525,6 +527,61 @@ struct Builder {
         return w;
     }
 
+    // The Bluestein (rader false) or Rader entries of this precision: conv_catalog.h, or bluestein_catalog.h
+    // (whose entries serve both) for plans that may run on the fused multi-pass kernels.
+    std::vector<BlueEntry> conv_choices(bool rader) {
+        std::vector<BlueEntry> out;
+        int count = 0;
+        const BlueEntry* old = blue_entries(&count);
+        if (req.fused_passes) {
+            for (int i = 0; i < count; ++i)
+                if (old[i].dbl == (req.dbl ? 1 : 0)) out.push_back(old[i]);
+            return out;
+        }
+        for (int i = 0; const ConvEntry* c = conv_entry(i); ++i) {
+            if (c->dbl != (req.dbl ? 1 : 0) || (c->rader != 0) != rader) continue;
+            if (static_cast<int64_t>(c->w) * c->pitch * cs > smem_limit) continue;
+            BlueEntry e{count + c->id, c->dbl, c->kind, c->n, c->tpl, c->w, c->maxt, {}, c->nstages};
+            std::copy(c->radices, c->radices + c->nstages, e.radices);
+            out.push_back(e);
+        }
+        return out;
+    }
+
+    // Kernel and twiddles of a pass on entry `e` of conv_choices.
+    void use_conv(PassSpec& ps, const BlueEntry& e) {
+        int count = 0;
+        blue_entries(&count);
+        ps.blue_id = e.id;
+        ps.blue_kind = e.kind;
+        if (e.id < count) return;
+        ps.conv_id = e.id - count;
+        const ConvEntry& c = *conv_entry(ps.conv_id);
+        std::vector<int> key(c.radices, c.radices + c.nstages);
+        const bool pair = c.kind == kBlueFused || c.kind == kBlueRowsConv;
+        key.push_back(pair ? -3 : -2);  // -2: the table of smooth_table
+        auto it = seq_tables.find(key);
+        if (it == seq_tables.end()) it = seq_tables.emplace(key, add_table(conv_twiddles(c))).first;
+        ps.tables.smooth = it->second;
+    }
+
+    // What a convolution of `points` points takes on these entries: their timed cost per point, or (entries
+    // of bluestein_catalog.h) the points alone.
+    double conv_time(int64_t points, std::initializer_list<const BlueEntry*> es) {
+        int count = 0;
+        blue_entries(&count);
+        double c = 0;
+        for (const BlueEntry* e : es) c += e->id < count ? 1.0 : conv_entry(e->id - count)->cost;
+        return c * static_cast<double>(points);
+    }
+
+    // The inverse column kernel of a length.
+    static const BlueEntry* inverse_of(const std::vector<BlueEntry>& cat, const BlueEntry& fwd) {
+        for (const BlueEntry& e : cat)
+            if (e.kind == kBlueColsInv && e.n == fwd.n) return &e;
+        return nullptr;
+    }
+
     // Rader on the size-specialised Bluestein kernels (contiguous axes, prime L): with g a
     // primitive root mod L, X[g^-q] = x[0] + sum_{p<M} x[g^p] W^(g^(p-q)), M = L - 1, a cyclic
     // convolution of a[p] = x[g^p] with b[m] = W^(g^-m) (W = exp(sgn 2 pi i / L)). It runs on
@@ -536,8 +593,8 @@ struct Builder {
     bool rader_fixed(int ax, int64_t L, int64_t O, Buf& cur) {
         if (req.no_fixed || req.no_rader || L < 3 || L > (int64_t(1) << 30) || !is_prime(L)) return false;
         const int64_t M = L - 1;
-        int count = 0;
-        const BlueEntry* cat = blue_entries(&count);
+        const std::vector<BlueEntry> cat = conv_choices(true);
+        const int count = static_cast<int>(cat.size());
         const int ps_shift = pad_shift_for(req.dbl);
         const BlueEntry* fused = nullptr;
         for (int i = 0; i < count && !fused; ++i) {
@@ -546,24 +603,32 @@ struct Builder {
                 int64_t(kmode_pitch(e.n, ps_shift)) * cs <= smem_limit)
                 fused = &e;
         }
+        // three passes only where Bluestein would take three too (its one block reads and writes HBM once)
+        bool one_block = false;
+        if (!fused && !req.fused_passes)
+            for (const BlueEntry& e : conv_choices(false))
+                one_block = one_block || (e.kind == kBlueFused && e.n >= 2 * L - 2 &&
+                                          int64_t(kmode_pitch(e.n, ps_shift)) * cs <= smem_limit);
         const BlueEntry *cf = nullptr, *rc = nullptr, *ci = nullptr;
-        for (int i = 0; i < count && !fused; ++i) {
+        double least = 0;
+        for (int i = 0; i < count && !fused && !one_block; ++i) {
             const BlueEntry& a = cat[i];
-            if (a.dbl != (req.dbl ? 1 : 0) || a.kind != kBlueColsFwd || M % a.n) continue;
-            if (int64_t(a.n) * a.w * cs > smem_limit) continue;
-            for (int k = 0; k < count; ++k) {
+            if (a.kind != kBlueColsFwd || M % a.n || int64_t(a.n) * a.w * cs > smem_limit) continue;
+            const BlueEntry* inv = inverse_of(cat, a);
+            for (int k = 0; k < count && inv; ++k) {
                 const BlueEntry& b = cat[k];
-                if (b.dbl != (req.dbl ? 1 : 0) || b.kind != kBlueRowsConv || int64_t(a.n) * b.n != M) continue;
+                if (b.kind != kBlueRowsConv || int64_t(a.n) * b.n != M) continue;
                 if (int64_t(kmode_pitch(b.n, ps_shift)) * cs > smem_limit) continue;
-                if (!cf || std::abs(std::log(double(b.n) / a.n)) < std::abs(std::log(double(rc->n) / cf->n))) {
+                const double t = conv_time(M, {&a, &b, inv});
+                if (!cf || t < least ||
+                    (t == least && std::abs(std::log(double(b.n) / a.n)) < std::abs(std::log(double(rc->n) / cf->n)))) {
+                    least = t;
                     cf = &a;
                     rc = &b;
+                    ci = inv;
                 }
             }
         }
-        if (cf)
-            for (int i = 0; i < count; ++i)
-                if (cat[i].dbl == cf->dbl && cat[i].kind == kBlueColsInv && cat[i].n == cf->n) ci = &cat[i];
         if (!fused && !(cf && rc && ci)) return false;
 
         const int sgn = req.direction;
@@ -625,8 +690,7 @@ struct Builder {
             ps.threads = round_up(p.w * p.tpl, 32);
             ps.smem_bytes = static_cast<int64_t>(p.w) * p.pitch * cs;
             ps.kc.maxt = fused->maxt;
-            ps.blue_id = fused->id;
-            ps.blue_kind = kBlueFused;
+            use_conv(ps, *fused);
             ps.rader = true;
             ps.src = cur;
             ps.dst = Buf::Output;
@@ -653,8 +717,7 @@ struct Builder {
             a.threads = round_up(e.w * e.tpl, 32);
             a.smem_bytes = static_cast<int64_t>(e.w) * n1 * cs;
             a.kc.maxt = e.maxt;
-            a.blue_id = e.id;
-            a.blue_kind = e.kind;
+            use_conv(a, e);
             a.rader = true;
         };
         // pass 1: columns of the gathered line a[p] = x[g^p]; W_M^(k1*c) on the store
@@ -707,8 +770,7 @@ struct Builder {
             b.threads = round_up(p.w * p.tpl, 32);
             b.smem_bytes = static_cast<int64_t>(p.w) * p.pitch * cs;
             b.kc.maxt = rc->maxt;
-            b.blue_id = rc->id;
-            b.blue_kind = kBlueRowsConv;
+            use_conv(b, *rc);
             b.rader = true;
             b.rader_dc = true;
             b.rader_src = cur;
@@ -738,14 +800,14 @@ struct Builder {
         return true;
     }
 
-    // Bluestein on the size-specialised kernels (contiguous axes): the smallest catalog
-    // convolution length M >= 2L - 2 (bluestein_length), as one fused pass where a fused
+    // Bluestein on the size-specialised kernels (contiguous axes): the catalog
+    // convolution length M >= 2L - 2 (bluestein_length) that takes the least time, as one fused pass where a fused
     // kernel of length M fits a CTA, else as M = n1 * n2 over a column kernel (n1) and a row
     // kernel (n2) in three passes. Returns false (generic kernels) when the catalog has no such length.
     bool bluestein_fixed(int ax, int64_t L, int64_t O, Buf& cur) {
         if (req.no_fixed) return false;
-        int count = 0;
-        const BlueEntry* cat = blue_entries(&count);
+        const std::vector<BlueEntry> cat = conv_choices(false);
+        const int count = static_cast<int>(cat.size());
         const int64_t need = 2 * L - 2;
         const int ps_shift = pad_shift_for(req.dbl);
         const BlueEntry* fused = nullptr;
@@ -753,33 +815,31 @@ struct Builder {
             const BlueEntry& e = cat[i];
             if (e.dbl != (req.dbl ? 1 : 0) || e.kind != kBlueFused || e.n < need) continue;
             if (int64_t(kmode_pitch(e.n, ps_shift)) * cs > smem_limit) continue;
-            if (!fused || e.n < fused->n) fused = &e;
+            if (!fused || conv_time(e.n, {&e}) < conv_time(fused->n, {fused})) fused = &e;
         }
-        const BlueEntry *cf = nullptr, *rc = nullptr;
+        const BlueEntry *cf = nullptr, *rc = nullptr, *ci = nullptr;
         int64_t best = 0;
+        double least = 0;
         for (int i = 0; i < count && !fused; ++i) {
             const BlueEntry& a = cat[i];
-            if (a.dbl != (req.dbl ? 1 : 0) || a.kind != kBlueColsFwd) continue;
-            if (int64_t(a.n) * a.w * cs > smem_limit) continue;
-            for (int k = 0; k < count; ++k) {
+            if (a.kind != kBlueColsFwd || int64_t(a.n) * a.w * cs > smem_limit) continue;
+            const BlueEntry* inv = inverse_of(cat, a);
+            for (int k = 0; k < count && inv; ++k) {
                 const BlueEntry& b = cat[k];
-                if (b.dbl != (req.dbl ? 1 : 0) || b.kind != kBlueRowsConv) continue;
+                if (b.kind != kBlueRowsConv) continue;
                 const int64_t M = int64_t(a.n) * b.n;
                 if (M < need || int64_t(kmode_pitch(b.n, ps_shift)) * cs > smem_limit) continue;
-                const bool better = !cf || M < best ||
-                                    (M == best && std::abs(std::log(double(b.n) / a.n)) <
-                                                      std::abs(std::log(double(rc->n) / cf->n)));
-                if (better) {
+                const double t = conv_time(M, {&a, &b, inv});
+                if (!cf || t < least ||
+                    (t == least && std::abs(std::log(double(b.n) / a.n)) < std::abs(std::log(double(rc->n) / cf->n)))) {
+                    least = t;
                     best = M;
                     cf = &a;
                     rc = &b;
+                    ci = inv;
                 }
             }
         }
-        const BlueEntry* ci = nullptr;
-        if (cf)
-            for (int i = 0; i < count; ++i)
-                if (cat[i].dbl == cf->dbl && cat[i].kind == kBlueColsInv && cat[i].n == cf->n) ci = &cat[i];
         if (!fused && !(cf && rc && ci)) return false;
 
         const bool bwd = req.direction == 1;
@@ -827,8 +887,7 @@ struct Builder {
             ps.threads = round_up(p.w * p.tpl, 32);
             ps.smem_bytes = static_cast<int64_t>(p.w) * p.pitch * cs;
             ps.kc.maxt = fused->maxt;
-            ps.blue_id = fused->id;
-            ps.blue_kind = kBlueFused;
+            use_conv(ps, *fused);
             ps.src = cur;
             ps.dst = Buf::Output;
             ps.bytes_moved = 2 * E * cs;
@@ -870,8 +929,7 @@ struct Builder {
             a.threads = round_up(e.w * e.tpl, 32);
             a.smem_bytes = static_cast<int64_t>(e.w) * n1 * cs;
             a.kc.maxt = e.maxt;
-            a.blue_id = e.id;
-            a.blue_kind = e.kind;
+            use_conv(a, e);
         };
         // pass 1: columns of the zero-padded, chirp-multiplied line; W_M^(k1*c) on the store
         PassSpec a;
@@ -923,8 +981,7 @@ struct Builder {
             b.threads = round_up(p.w * p.tpl, 32);
             b.smem_bytes = static_cast<int64_t>(p.w) * p.pitch * cs;
             b.kc.maxt = rc->maxt;
-            b.blue_id = rc->id;
-            b.blue_kind = kBlueRowsConv;
+            use_conv(b, *rc);
             b.src = Buf::Scratch;
             b.dst = Buf::Scratch;
             b.bytes_moved = 2 * O * M * cs;
@@ -1649,20 +1706,52 @@ const SmoothEntry* find_smooth(bool dbl, int kind, int feat, int n) {
     return it == index.end() ? nullptr : it->second;
 }
 
-std::vector<std::complex<double>> smooth_twiddles(const SmoothEntry& e) {
-    std::vector<int64_t> key(e.radices, e.radices + e.nstages);
+namespace {
+// Per stage the rows W_(ns*R)^(r*jm), jm < ns, for r = 1, 2, 4, 8 below R.
+std::vector<std::complex<double>> stage_rows(const std::vector<int>& radices) {
+    std::vector<int64_t> key(radices.begin(), radices.end());
     key.push_back(-600);
     return *cached_table(key, [&] {
         std::vector<std::complex<double>> t;
         int64_t ns = 1;
-        for (int s = 0; s < e.nstages; ++s) {
-            const int R = e.radices[s];
+        for (int R : radices) {
             for (int q = 0; q < smooth_tw_entries(R); ++q)
                 for (int64_t jm = 0; jm < ns; ++jm) t.push_back(cis_neg((int64_t(1) << q) * jm, ns * R));
             ns *= R;
         }
         return t;
     });
+}
+
+const std::vector<ConvEntry>& all_conv_entries() {
+    static const std::vector<ConvEntry> all = {
+#define SFB_X(ID, DBL, KIND, RADER, N, TPL, W, PADS, PITCH, MAXT, MINB, COST, ...) \
+    {ID, DBL, KIND, RADER, N, TPL, W, PADS, PITCH, MAXT, MINB, COST, {__VA_ARGS__}, count_args(__VA_ARGS__)},
+        SFB_CONV_CATALOG(SFB_X)
+#undef SFB_X
+    };
+    return all;
+}
+}  // namespace
+
+std::vector<std::complex<double>> smooth_twiddles(const SmoothEntry& e) {
+    return stage_rows(std::vector<int>(e.radices, e.radices + e.nstages));
+}
+
+const ConvEntry* conv_entry(int id) {
+    const auto& all = all_conv_entries();
+    return id >= 0 && id < static_cast<int>(all.size()) ? &all[id] : nullptr;
+}
+
+std::vector<std::complex<double>> conv_twiddles(const ConvEntry& e) {
+    std::vector<int> r(e.radices, e.radices + e.nstages);
+    auto t = stage_rows(r);
+    if (e.kind == kBlueFused || e.kind == kBlueRowsConv) {
+        std::reverse(r.begin(), r.end());
+        const auto back = stage_rows(r);
+        t.insert(t.end(), back.begin(), back.end());
+    }
+    return t;
 }
 
 int strided_line_kind(const LineLayout& in, const LineLayout& out) {

@@ -83,6 +83,9 @@ struct PassSpec {
     // size-specialised kernel of the 7-smooth lengths (smooth_catalog.h) that runs this pass in place of
     // the kernel named above, with its own stage sequence (table tables.smooth); -1: none
     int smooth_id = -1;
+    // Bluestein / Rader pass on a conv_catalog.h kernel (blue_id is then past the ids of bluestein_catalog.h;
+    // the twiddles are tables.smooth); -1: on the kernel of blue_id
+    int conv_id = -1;
 };
 
 // The lean kernel's instantiations (lean_variants.cu): float with 16 values per thread, double
@@ -145,6 +148,21 @@ struct BlueEntry {
 };
 const BlueEntry* blue_entries(int* count);
 
+// One entry of conv_catalog.h: a Bluestein (rader 0) or Rader pass kernel of conv_kernel.cuh; kind as above.
+struct ConvEntry {
+    int id, dbl, kind, rader, n, tpl, w, pads, pitch, maxt, minb;
+    int cost;  // time per point of the convolution, 10 fs (timed on B200, the whole chip busy)
+    int radices[kMaxStages];
+    int nstages;
+};
+const ConvEntry* conv_entry(int id);
+// Shared memory of a column scatter's indices.
+inline int64_t conv_index_bytes(const ConvEntry& e) {
+    return e.rader && e.kind == kBlueColsInv ? int64_t(e.n) * e.w * 4 : 0;
+}
+// Its stage twiddles: the rows of smooth_twiddles over its radices, then (convolutions) over the reverse.
+std::vector<std::complex<double>> conv_twiddles(const ConvEntry& e);
+
 // One entry of tc_catalog.h (split-precision tensor-core kernels, complex<float> only).
 struct TcEntry {
     int id, r, s, l, cols;
@@ -191,6 +209,8 @@ struct PlanRequest {
     // smooth_catalog.h kernel of the two mappings (strided_line_kind).
     bool strided_line = false;
     LineLayout line_in, line_out;
+    // the fused multi-pass kernels may run the plan (an opt-in): Bluestein passes on bluestein_catalog.h
+    bool fused_passes = false;
     // prime lengths L take Bluestein's convolution even where the catalog covers L - 1 (Rader)
     bool no_rader = false;
 };

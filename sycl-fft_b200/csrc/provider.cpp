@@ -28,6 +28,7 @@
 #include "launch.hpp"
 #include "lean_launch.hpp"
 #include "smooth_launch.hpp"
+#include "conv_launch.hpp"
 #include "piped_launch.hpp"
 #include "tc_launch.hpp"
 #include "tma_launch.hpp"
@@ -92,6 +93,7 @@ struct BoundPass {
     const FusedBlueEntry* fusedblue = nullptr;
     const SmoothEntry* smooth = nullptr;  // size-specialised kernel of a 7-smooth length, and its twiddles
     const void* smooth_tw = nullptr;
+    const ConvEntry* conv = nullptr;      // or the conv_catalog.h kernel of a Bluestein / Rader pass
 };
 
 TcParams to_tc(const PassParams& p, const void* tw, int* status) {
@@ -475,6 +477,7 @@ DevicePlan* create_plan(const syclfft_b200_plan_config_v1& cfg, uint32_t flags, 
     if (const char* k = std::getenv("SYCLFFT_B200_FUSED4_SINGLE")) req.fused_single = std::strcmp(k, "1") == 0;
     if (const char* k = std::getenv("SYCLFFT_B200_FUSED4")) {
         if (std::strcmp(k, "1") != 0) req.fused_single = false;
+        req.fused_passes = std::strcmp(k, "1") == 0;
     } else {
         req.fused_single = false;  // the fused kernels are opt-in
     }
@@ -518,14 +521,15 @@ DevicePlan* build_plan(PlanRequest req, int device, uint32_t flags, const std::s
 
     // All tables in one allocation, each 256-byte aligned: the complex tables (cast to the
     // plan precision), then the int32 index tables.
-    // A pass on a smooth_catalog.h kernel reads that kernel's stage table instead of tw1 (unless the fused
+    // A pass on a smooth_catalog.h or conv_catalog.h kernel reads that kernel's stage table instead of tw1, tw2 (unless the fused
     // multi-pass kernels, an opt-in, take it): tables no kernel reads are not uploaded.
     const char* f4env = std::getenv("SYCLFFT_B200_FUSED4");
     const bool fused_opt_in = f4env && f4env[0] == '1';
     std::vector<char> read(plan->spec.tables.size(), fused_opt_in ? 1 : 0);
     for (const PassSpec& ps : plan->spec.passes) {
         const TableIds& t = ps.tables;
-        for (int id : {ps.smooth_id >= 0 ? -1 : t.tw1, t.tw2, t.premul, t.pointwise, t.postmul, t.tw4_hi, t.tw4_lo, t.tc_tw,
+        const bool own = ps.smooth_id >= 0 || ps.conv_id >= 0;
+        for (int id : {own ? -1 : t.tw1, own ? -1 : t.tw2, t.premul, t.pointwise, t.postmul, t.tw4_hi, t.tw4_lo, t.tc_tw,
                        t.cl_base, t.smooth})
             if (id >= 0) read[id] = 1;
     }
@@ -638,6 +642,7 @@ DevicePlan* build_plan(PlanRequest req, int device, uint32_t flags, const std::s
         bp.tp = to_tc(bp.p, tab(ps.tables.tc_tw), plan->status);
         bp.smooth = smooth_entry(ps.smooth_id);
         bp.smooth_tw = tab(ps.tables.smooth);
+        bp.conv = conv_entry(ps.conv_id);
         plan->passes.push_back(bp);
     }
     // four-step column + row passes (and Bluestein's three passes) of a contiguous axis with a
@@ -1269,6 +1274,10 @@ void launch_bound_pass(DevicePlan* plan, const BoundPass& bp, void* src, void* d
         int64_t n_outer = 1;
         const SmoothParams sp = to_smooth(bp.p, bp.smooth_tw, &n_outer);
         check(launch_smooth(*bp.smooth, sp, n_outer, plan->sms, src, dst, stream), "FFT pass launch");
+    } else if (bp.conv) {
+        FixedParams fp = bp.fp;
+        fp.tw = bp.smooth_tw;
+        check(launch_conv(*bp.conv, fp, bp.p.n_outer, plan->sms, src, dst, stream), "FFT convolution pass launch");
     } else if (ps.blue_id >= 0) {
         check(launch_blue(ps.blue_id, plan->spec.req.dbl, ps.blue_kind, ps.rader, bp.fp, ps.threads,
                           static_cast<size_t>(ps.smem_bytes), bp.p.tiles, src, dst, stream),

@@ -13,8 +13,8 @@ from native_libs import butterfly, describe, real_pair, smooth_run, smooth_run_l
 KK, CC, CK, KC = 0, 1, 2, 3
 
 
-def catalog():
-    src = open(os.path.join(os.path.dirname(__file__), "..", "sycl-fft_b200", "csrc", "smooth_catalog.h")).read()
+def catalog(name="smooth_catalog.h"):
+    src = open(os.path.join(os.path.dirname(__file__), "..", "sycl-fft_b200", "csrc", name)).read()
     return [tuple(int(v) for v in m.split(",")) for m in re.findall(r"X\(([-0-9, ]+)\)", src)]
 
 
@@ -42,6 +42,19 @@ def test_catalog_geometry():
         assert feat in (0, {KK: 0, CC: 1}.get(kind, 0)) or (kind == KK and feat in (2, 4)), e
 
 
+def test_convolution_catalog_geometry():
+    entries = catalog("conv_catalog.h")
+    assert [e[0] for e in entries] == list(range(len(entries)))
+    assert len({e[1:5] for e in entries}) == len(entries)
+    for e in entries:
+        _, dbl, kind, rader, n, tpl, w, pads, pitch, maxt, minb, cost, *radices = e
+        assert np.prod(radices) == n and len(radices) >= 2 and max(radices) <= 16, e
+        assert (w * tpl + 31) // 32 * 32 == maxt <= 1024 and maxt * minb <= 2048, e
+        assert pitch > (n - 1) + ((n - 1) >> pads if pads else 0), e
+        assert w * pitch * (16 if dbl else 8) <= 227 * 1024, e
+        assert kind in (0, 2) or w & (w - 1) == 0, e
+
+
 # the shortest and longest lines of each mapping, one with idle threads in a stage, several lines per block
 @pytest.mark.parametrize("double", [False, True])
 @pytest.mark.parametrize("shape,batch", [([18], 70), ([45], 97), ([105], 25), ([810], 3), ([1029], 2), ([3000], 2),
@@ -55,6 +68,23 @@ def test_contiguous_plans_by_thread(shape, batch, double):
         if y is None:
             pytest.skip("a pass of this plan is not a 7-smooth kernel")
         assert rel_l2(y, fp64_fft(x, shape, batch, d, norm_scale(norm, d, n))) < 1e-13
+
+
+# fused and three-pass Bluestein (the shortest and longest block, the first three-pass lengths), Rader in
+# one block and in three passes, a prime axis of a grid
+@pytest.mark.parametrize("n,batch,double", [
+    ([11], 40, False), ([11], 40, True), ([37], 9, True), ([509], 3, True), ([1009], 2, False), ([4099], 1, False),
+    ([4099], 1, True), ([8191], 1, False), ([8209], 1, False), ([3583], 1, True), ([257], 5, False), ([641], 3, True),
+    ([12289], 1, True), ([19, 17], 2, False),
+], ids=str)
+def test_convolutions_by_thread(n, batch, double):
+    total = int(np.prod(n))
+    x = gaussian_complex(total * batch, total + batch, np.complex128)
+    for d, norm, ip in ((-1, 1, False), (1, 2, True)):
+        y = smooth_run(x, n, batch, d, norm, double, ip)
+        if y is None:
+            pytest.skip("a pass of this plan is on the general kernel")
+        assert rel_l2(y, fp64_fft(x, n, batch, d, norm_scale(norm, d, total))) < 1e-13
 
 
 @pytest.mark.parametrize("w_lines", [1, 2, 3])
@@ -102,6 +132,15 @@ def test_dispatch():
     assert ids([840, 1200]) == [True, True]
     assert ids([256, 256], split_bf16=True) == [False, False]
     assert ids([1009]) == [False]
+
+
+def test_three_pass_split():
+    """A split convolution is at least 2L - 2 long and not much longer: the pair of catalog lengths whose
+    passes take the least time."""
+    for n, dbl in ((40009, False), (65521, True), (8209, True), (300007, False)):
+        p = describe([n], 2, double=dbl)["passes"]
+        assert [x["kind"] for x in p] == ["bluestein_cols_fwd", "bluestein_rows_conv", "bluestein_cols_inv"]
+        assert 2 * n - 2 <= p[0]["n"] * p[1]["n"] < 1.25 * (2 * n - 2)
 
 
 @pytest.mark.parametrize("n", [1, 6, 15])
