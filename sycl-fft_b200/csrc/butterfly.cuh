@@ -1,4 +1,4 @@
-// Register-resident forward DFT butterflies of radix 1 to 10, 12, 14, 15 and 16.
+// Register-resident forward DFT butterflies of radix 1 to 10, 12, 14 to 16, 18, 20, 21, 24, 25, 27, 28, 30 and 32.
 //
 // All butterflies compute X_p = sum_q v_q * exp(-2*pi*i*p*q/R) in place on an array
 // of R complex values held in registers. Inverse transforms are obtained by the
@@ -64,6 +64,46 @@ template <class C> SFB_HD C cmake(decltype(C::x) x, decltype(C::x) y) { C r; r.x
 #define SFB_K9C4 -0.939692620785908384054
 #define SFB_K9S4 0.342020143325668733044
 #define SFB_K8 0.707106781186547524401
+#define SFB_K32C1 0.980785280403230449126
+#define SFB_K32S1 0.195090322016128267848
+#define SFB_K32C3 0.831469612302545237079
+#define SFB_K32S3 0.555570233019602224743
+#define SFB_K25C1 0.968583161128631119490
+#define SFB_K25S1 0.248689887164854788242
+#define SFB_K25C2 0.876306680043863587308
+#define SFB_K25S2 0.481753674101715274987
+#define SFB_K25C3 0.728968627421411523147
+#define SFB_K25S3 0.684547105928688673732
+#define SFB_K25C4 0.535826794978996618271
+#define SFB_K25S4 0.844327925502015078549
+#define SFB_K25C6 0.0627905195293133760762
+#define SFB_K25S6 0.998026728428271561952
+#define SFB_K25C8 -0.425779291565072648863
+#define SFB_K25S8 0.904827052466019527714
+#define SFB_K25C9 -0.637423989748689710177
+#define SFB_K25S9 0.770513242775789230803
+#define SFB_K25C12 -0.992114701314477831050
+#define SFB_K25S12 0.125333233564304245373
+#define SFB_K25C16 -0.637423989748689710177
+#define SFB_K25S16 -0.770513242775789230803
+#define SFB_K27C1 0.973044870579823838833
+#define SFB_K27S1 0.230615870742440178450
+#define SFB_K27C2 0.893632640323412248193
+#define SFB_K27S2 0.448799180200462172785
+#define SFB_K27C4 0.597158591702786164852
+#define SFB_K27S4 0.802123192755043785083
+#define SFB_K27C5 0.396079766039156823696
+#define SFB_K27S5 0.918216106880274014759
+#define SFB_K27C7 -0.0581448289104758285387
+#define SFB_K27S7 0.998308158271268208048
+#define SFB_K27C8 -0.286803232711090253103
+#define SFB_K27S8 0.957989512315488874437
+#define SFB_K27C10 -0.686241637868733585730
+#define SFB_K27S10 0.727373641573048695987
+#define SFB_K27C14 -0.993238357741942988548
+#define SFB_K27S14 -0.116092914125230229676
+#define SFB_K27C16 -0.835487811412936419654
+#define SFB_K27S16 -0.549508978070806035263
 #define SFB_K16C 0.923879532511286756128
 #define SFB_K16S 0.382683432365089771728
 
@@ -265,6 +305,88 @@ template <class T, class C> SFB_HD void bfly9(C* v) {
     }
 }
 
+// Radix A * B in two steps: n = n2 + B*n1, A-point DFTs over n1, the constant twiddles W_AB^(n2*k1), B-point
+// DFTs over n2; X[k1 + A*k2]. `w` holds (cos, sin) of 2 pi m / AB at index m.
+template <int A, int B, class T, class C, class W> SFB_HD void bfly_two(C* v, W w) {
+    C a[B][A];
+#pragma unroll
+    for (int n2 = 0; n2 < B; ++n2) {
+#pragma unroll
+        for (int n1 = 0; n1 < A; ++n1) a[n2][n1] = v[n2 + B * n1];
+        dft<A, T>(a[n2]);
+#pragma unroll
+        for (int k1 = 1; k1 < A; ++k1)
+            if (n2 > 0) a[n2][k1] = w(n2 * k1, a[n2][k1]);
+    }
+#pragma unroll
+    for (int k1 = 0; k1 < A; ++k1) {
+        C b[B];
+#pragma unroll
+        for (int n2 = 0; n2 < B; ++n2) b[n2] = a[n2][k1];
+        dft<B, T>(b);
+#pragma unroll
+        for (int k2 = 0; k2 < B; ++k2) v[k1 + A * k2] = b[k2];
+    }
+}
+
+template <class T> struct Twiddle25 {
+    template <class C> SFB_HD C operator()(int m, C a) const {
+        switch (m) {
+            case 1: return cmul(a, cmake<C>(T(SFB_K25C1), T(-SFB_K25S1)));
+            case 2: return cmul(a, cmake<C>(T(SFB_K25C2), T(-SFB_K25S2)));
+            case 3: return cmul(a, cmake<C>(T(SFB_K25C3), T(-SFB_K25S3)));
+            case 4: return cmul(a, cmake<C>(T(SFB_K25C4), T(-SFB_K25S4)));
+            case 6: return cmul(a, cmake<C>(T(SFB_K25C6), T(-SFB_K25S6)));
+            case 8: return cmul(a, cmake<C>(T(SFB_K25C8), T(-SFB_K25S8)));
+            case 9: return cmul(a, cmake<C>(T(SFB_K25C9), T(-SFB_K25S9)));
+            case 12: return cmul(a, cmake<C>(T(SFB_K25C12), T(-SFB_K25S12)));
+            default: return cmul(a, cmake<C>(T(SFB_K25C16), T(-SFB_K25S16)));
+        }
+    }
+};
+
+template <class T> struct Twiddle27 {
+    template <class C> SFB_HD C operator()(int m, C a) const {
+        switch (m) {
+            case 1: return cmul(a, cmake<C>(T(SFB_K27C1), T(-SFB_K27S1)));
+            case 2: return cmul(a, cmake<C>(T(SFB_K27C2), T(-SFB_K27S2)));
+            case 3: return cmul(a, cmake<C>(T(SFB_K9C1), T(-SFB_K9S1)));
+            case 4: return cmul(a, cmake<C>(T(SFB_K27C4), T(-SFB_K27S4)));
+            case 5: return cmul(a, cmake<C>(T(SFB_K27C5), T(-SFB_K27S5)));
+            case 6: return cmul(a, cmake<C>(T(SFB_K9C2), T(-SFB_K9S2)));
+            case 7: return cmul(a, cmake<C>(T(SFB_K27C7), T(-SFB_K27S7)));
+            case 8: return cmul(a, cmake<C>(T(SFB_K27C8), T(-SFB_K27S8)));
+            case 10: return cmul(a, cmake<C>(T(SFB_K27C10), T(-SFB_K27S10)));
+            case 12: return cmul(a, cmake<C>(T(SFB_K9C4), T(-SFB_K9S4)));
+            case 14: return cmul(a, cmake<C>(T(SFB_K27C14), T(-SFB_K27S14)));
+            default: return cmul(a, cmake<C>(T(SFB_K27C16), T(-SFB_K27S16)));
+        }
+    }
+};
+
+template <class T> struct Twiddle32 {
+    template <class C> SFB_HD C operator()(int m, C a) const {
+        const T k = T(SFB_K8);
+        switch (m) {
+            case 1: return cmul(a, cmake<C>(T(SFB_K32C1), T(-SFB_K32S1)));
+            case 2: return cmul(a, cmake<C>(T(SFB_K16C), T(-SFB_K16S)));
+            case 3: return cmul(a, cmake<C>(T(SFB_K32C3), T(-SFB_K32S3)));
+            case 4: return cmake<C>(k * (a.x + a.y), k * (a.y - a.x));
+            case 5: return cmul(a, cmake<C>(T(SFB_K32S3), T(-SFB_K32C3)));
+            case 6: return cmul(a, cmake<C>(T(SFB_K16S), T(-SFB_K16C)));
+            case 7: return cmul(a, cmake<C>(T(SFB_K32S1), T(-SFB_K32C1)));
+            case 8: return cmul_mi(a);
+            case 9: return cmul(a, cmake<C>(T(-SFB_K32S1), T(-SFB_K32C1)));
+            case 10: return cmul(a, cmake<C>(T(-SFB_K16S), T(-SFB_K16C)));
+            case 12: return cmake<C>(k * (a.y - a.x), -k * (a.x + a.y));
+            case 14: return cmul(a, cmake<C>(T(-SFB_K16C), T(-SFB_K16S)));
+            case 15: return cmul(a, cmake<C>(T(-SFB_K32C1), T(-SFB_K32S1)));
+            case 18: return cmul(a, cmake<C>(T(-SFB_K16C), T(SFB_K16S)));
+            default: return cmul(a, cmake<C>(T(-SFB_K32S3), T(SFB_K32C3)));  // 21
+        }
+    }
+};
+
 // u[r] *= w^r for r = 1..R-1, the powers formed by a balanced product tree
 // (w^r = w^h * w^(r-h), h the largest power of two <= r): at most log2(R)+1 roundings deep.
 template <int R, class C> SFB_HD void twiddle_powers(C* u, C w) {
@@ -335,6 +457,25 @@ template <int R, class T, class C> SFB_HD void dft(C* v) {
         bfly15<T>(v);
     } else if constexpr (R == 16) {
         bfly16<T>(v);
+    } else if constexpr (R == 18) {
+        bfly_pfa<2, 9, T>(v);
+    } else if constexpr (R == 20) {
+        bfly_pfa<4, 5, T>(v);
+    } else if constexpr (R == 21) {
+        bfly_pfa<3, 7, T>(v);
+    } else if constexpr (R == 24) {
+        bfly_pfa<3, 8, T>(v);
+    } else if constexpr (R == 25) {
+        bfly_two<5, 5, T>(v, Twiddle25<T>());
+    } else if constexpr (R == 27) {
+        bfly_two<9, 3, T>(v, Twiddle27<T>());
+    } else if constexpr (R == 28) {
+        bfly_pfa<4, 7, T>(v);
+    } else if constexpr (R == 30) {
+        bfly_pfa<2, 15, T>(v);
+    } else {
+        static_assert(R == 32, "no butterfly of this radix");
+        bfly_two<8, 4, T>(v, Twiddle32<T>());
     }
 }
 

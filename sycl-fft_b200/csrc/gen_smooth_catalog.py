@@ -12,23 +12,26 @@ a bank simulation of every exchange, and the bytes in flight of the blocks that 
 first choices are within 10% of the fastest on average and up to 2x off for single lengths, so the
 committed catalog holds the fastest of 20,000 candidates timed on B200 (128 MB of input each). A
 complex length is left out where the power-of-two kernel of fixed_catalog.h was faster (64-point float
-lines). The real transforms (FEAT 2 and 4) take the layouts chosen for complex lines.
+lines). The real transforms (FEAT 2 and 4) take the layouts chosen for complex lines, or one with a radix
+above 16 where that was faster for them. Radices above 16 (float only: a double butterfly of 18 values takes
+more than 128 registers) are taken where they timed at least 1.5% below the best layout of radices to 16.
 """
 import itertools
 import math
 import sys
 
 KK, CC, CK, KC = 0, 1, 2, 3
-RADICES = (2, 3, 4, 5, 6, 7, 8, 9, 10, 12, 14, 15, 16)
+RADICES = (2, 3, 4, 5, 6, 7, 8, 9, 10, 12, 14, 15, 16, 18, 20, 21, 24, 25, 27, 28, 30, 32)
 # floating-point instructions of one butterfly (adds, multiplies, fused multiply-adds)
-FP = {2: 4, 3: 14, 4: 16, 5: 40, 6: 40, 7: 78, 8: 56, 9: 104, 10: 100, 12: 104, 14: 184, 15: 190, 16: 160}
-TW_LOADS = {r: (4 if r > 8 else 3 if r > 4 else 2 if r > 2 else 1) for r in RADICES}
+FP = {2: 4, 3: 14, 4: 16, 5: 40, 6: 40, 7: 78, 8: 56, 9: 104, 10: 100, 12: 104, 14: 184, 15: 190, 16: 160,
+      18: 244, 20: 240, 21: 332, 24: 280, 25: 464, 27: 502, 28: 424, 30: 440, 32: 430}
+TW_LOADS = {r: (5 if r > 16 else 4 if r > 8 else 3 if r > 4 else 2 if r > 2 else 1) for r in RADICES}
 SMEM = 227 * 1024
 
 
 def max_values(dbl, kind, n):
-    """Complex values a thread may hold: long float lines need more than 16 to fit 1024 threads."""
-    return 32 if not dbl and kind == KK and n > 6144 else 16
+    """Complex values a thread may hold: 32 float values (radices above 16) take up to 128 registers."""
+    return 16 if dbl else 32
 
 
 KEEP = 8  # candidates per entry that are timed
@@ -41,7 +44,7 @@ def smooth(n):
     return n == 1
 
 
-def multisets(n, stages, top=16):
+def multisets(n, stages, top=32):
     if stages == 1:
         return [(n,)] if n in RADICES and n <= top else []
     out = []
@@ -55,7 +58,7 @@ def regs(values, dbl):
     """Registers a thread needs for `values` complex values (observed, without spills)."""
     if dbl:
         return 64 if values <= 8 else 76 if values <= 10 else 92 if values <= 12 else 120
-    return 40 if values <= 8 else 48 if values <= 10 else 56 if values <= 16 else 72 if values <= 20 else 88 if values <= 25 else 120
+    return 40 if values <= 8 else 48 if values <= 10 else 56 if values <= 16 else 72 if values <= 20 else 96 if values <= 25 else 112 if values <= 28 else 128
 
 
 def conflicts(addr, per):

@@ -34,11 +34,13 @@ enum : int { kSmoothKK = 0, kSmoothCC = 1, kSmoothCK = 2, kSmoothKC = 3 };
 // Features of a smooth_kernel.cuh instantiation: four-step twiddle on the store; real transforms of length
 // 2N, bins formed after the last stage (R2C) or read before the first (C2R).
 enum : int { kSmoothTw4 = 1, kSmoothPost = 2, kSmoothPre = 4 };
-// Rows of a radix-R stage's twiddle table in smooth_kernel.cuh: W^(r*jm) for r = 1, 2, 4, 8 below R.
+// Rows of a radix-R stage's twiddle table in smooth_kernel.cuh: W^(r*jm) for r = 1, 2, 4, 8 below R; above
+// radix 16 for r = 1, 2, 3, 4, 8, 12, .. below R.
 #if defined(__CUDACC__)
 __host__ __device__
 #endif
-constexpr int smooth_tw_entries(int R) { return R > 8 ? 4 : R > 4 ? 3 : R > 2 ? 2 : 1; }
+constexpr int smooth_tw_entries(int R) { return R > 16 ? 3 + (R - 1) / 4 : R > 8 ? 4 : R > 4 ? 3 : R > 2 ? 2 : 1; }
+inline int smooth_tw_power(int R, int q) { return R <= 16 ? 1 << q : q < 3 ? q + 1 : 4 * (q - 2); }  // of row q
 enum : int { kSelNone = 0, kSelCol = 1, kSelOuterLo = 2, kSelColMod = 3 };
 
 struct LineLayout {

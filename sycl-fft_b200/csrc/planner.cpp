@@ -1707,7 +1707,7 @@ const SmoothEntry* find_smooth(bool dbl, int kind, int feat, int n) {
 }
 
 namespace {
-// Per stage the rows W_(ns*R)^(r*jm), jm < ns, for r = 1, 2, 4, 8 below R.
+// Per stage the rows W_(ns*R)^(r*jm), jm < ns, r = smooth_tw_power(R, row).
 std::vector<std::complex<double>> stage_rows(const std::vector<int>& radices) {
     std::vector<int64_t> key(radices.begin(), radices.end());
     key.push_back(-600);
@@ -1716,7 +1716,7 @@ std::vector<std::complex<double>> stage_rows(const std::vector<int>& radices) {
         int64_t ns = 1;
         for (int R : radices) {
             for (int q = 0; q < smooth_tw_entries(R); ++q)
-                for (int64_t jm = 0; jm < ns; ++jm) t.push_back(cis_neg((int64_t(1) << q) * jm, ns * R));
+                for (int64_t jm = 0; jm < ns; ++jm) t.push_back(cis_neg(smooth_tw_power(R, q) * jm, ns * R));
             ns *= R;
         }
         return t;

@@ -124,7 +124,7 @@ struct SmoothEntry {
     int nstages;
 };
 const SmoothEntry* find_smooth(bool dbl, int kind, int feat, int n);
-// Its stage twiddles: per stage the rows W_(ns*R)^(r*jm), jm < ns, for r = 1, 2, 4, 8 below R.
+// Its stage twiddles: per stage the rows W_(ns*R)^(r*jm), jm < ns, r = smooth_tw_power(R, row).
 std::vector<std::complex<double>> smooth_twiddles(const SmoothEntry& e);
 const SmoothEntry* smooth_entry(int id);
 // The mapping pair of a strided one-dimensional layout, or -1 when a side is neither contiguous lines nor

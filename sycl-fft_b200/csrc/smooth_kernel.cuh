@@ -10,13 +10,20 @@
 //    factors take three or four stages instead of five to seven; an odd radix first where there is one:
 //    its exchange then falls in distinct banks without padding, which saves the padding's address
 //    arithmetic in every stage (3000 points: [8, 15, 5, 5] padded 197 us, [15, 8, 5, 5] without 156 us).
+//  * float radices to 32 at up to 128 registers a thread: 256 to 1024 points in two stages, longer lines in
+//    three. Shared-memory traffic (the load/store pipe was 66 to 78% busy) and barriers fall with every
+//    exchange, and the values in flight per SM rise. [15, 8, 5, 5] -> [25, 10, 12]: 3000 x 16384 178 -> 151
+//    us; 810 x 840 four-step [9, 9, 10] and [15, 4, 14] -> [27, 30] and [30, 28]: 680400 x 64 360 -> 310 us;
+//    1024 columns -> rows [16, 8, 8] -> [32, 32]: 240 -> 209 us. 869 of the 2290 float entries, those that
+//    gained at least 1.5%: 1.15x (geometric mean). Packed two-value additions (add.f32x2) in their place
+//    gave nothing: the exchanges, not the arithmetic, fill the time.
 //  * up to 16 values a thread in double too, at 128 registers and half the threads: the same bytes in
 //    flight with one exchange less (2048 points: [8, 8, 8, 4] 180 us, [16, 16, 8] 168 us per 1.07 GB).
 //
 // What bounds it: HBM for the lines up to about 2000 points (4.9 to 6.4 of the 6.5 TB/s copy rate), the
 // issue slots and exchanges of the longer ones, one or two blocks of which fill an SM. Times per execute on
-// B200 against the runtime-length kernels: 3000 x 16384 float 337 -> 178 us, 680400 x 64 float (810 x 840
-// four-step) 638 -> 359 us, 840 x 1200 x 4 float 101 -> 34 us; complex<double> 65536 x 512 (256 x 256)
+// B200 against the runtime-length kernels: 3000 x 16384 float 337 -> 151 us, 680400 x 64 float (810 x 840
+// four-step) 638 -> 310 us, 840 x 1200 x 4 float 101 -> 34 us; complex<double> 65536 x 512 (256 x 256)
 // 415 -> 354 us against fixed_kernel.cuh. All 691 whole-line lengths above 15: 1.96x (geometric mean, 64 MB
 // batches), columns 2.3x, four-steps to 2^20 1.67x.
 #pragma once
@@ -86,6 +93,25 @@ __device__ __forceinline__ void smooth_twiddle(C* u, const C* __restrict__ tw, i
     }
 }
 
+// Radices above 16: the power 4h + s is one product of the rows w^(4h) and w^s (s = 1, 2, 3), so that no power
+// is more than one product away from the table and few of them are live beside the values. Against
+// products of w, w^2, w^4, w^8 and w^16 alone: 3000 x 16384 158 -> 151 us, 680400 x 64 323 -> 310 us.
+template <int R, int NS, class C>
+__device__ __forceinline__ void smooth_twiddle_wide(C* u, const C* __restrict__ tw, int jm) {
+    const C w1 = __ldg(tw + jm), w2 = __ldg(tw + NS + jm), w3 = __ldg(tw + 2 * NS + jm);
+    u[1] = cmul(u[1], w1);
+    u[2] = cmul(u[2], w2);
+    u[3] = cmul(u[3], w3);
+#pragma unroll
+    for (int h = 1; 4 * h < R; ++h) {
+        const C b = __ldg(tw + (2 + h) * NS + jm);
+        u[4 * h] = cmul(u[4 * h], b);
+        if (4 * h + 1 < R) u[4 * h + 1] = cmul(u[4 * h + 1], cmul(b, w1));
+        if (4 * h + 2 < R) u[4 * h + 2] = cmul(u[4 * h + 2], cmul(b, w2));
+        if (4 * h + 3 < R) u[4 * h + 3] = cmul(u[4 * h + 3], cmul(b, w3));
+    }
+}
+
 template <int PADS>
 __device__ __forceinline__ int smooth_idx(int k) {
     if constexpr (PADS == 0) return k;
@@ -136,8 +162,13 @@ __device__ __forceinline__ void smooth_tw4(C* u, const SmoothCtx<T>& X, int j) {
     for (int r = 0; r < R && r < 8; ++r) u[r] = cmul(u[r], q[r]);
     if constexpr (R > 8) {
         const C s = smooth_tw4_at(X, 8 * NR * X.sel);
+        C t = s;
 #pragma unroll
-        for (int r = 8; r < R; ++r) u[r] = cmul(u[r], cmul(q[r - 8], s));
+        for (int r = 8; r < R; ++r) {
+            if (r == 16) t = smooth_tw4_at(X, 16 * NR * X.sel);
+            if (r == 24) t = cmul(t, s);
+            u[r] = cmul(u[r], cmul(q[r & 7], t));
+        }
     }
 }
 
@@ -195,7 +226,8 @@ __device__ __forceinline__ void smooth_stage(SmoothCtx<T>& X) {
         if (act && (EXACT || i + 1 < NB || j < NR)) {
             C* u = &v[i * R];
             const int jm = LAST ? j : j % NS;
-            if constexpr (NS > 1) smooth_twiddle<R, NS>(u, X.tw + TWOFF, jm);
+            if constexpr (NS > 1 && R > 16) smooth_twiddle_wide<R, NS>(u, X.tw + TWOFF, jm);
+            else if constexpr (NS > 1) smooth_twiddle<R, NS>(u, X.tw + TWOFF, jm);
             dft<R, T>(u);
             if constexpr (LAST && (FEAT & kSmoothPost)) {
                 // over the elements this thread read; the bins are formed from pairs after a barrier

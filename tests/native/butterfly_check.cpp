@@ -28,6 +28,15 @@ static int dispatch(int radix, const T* in, T* out) {
         case 14: run<14, T>(in, out); return 0;
         case 15: run<15, T>(in, out); return 0;
         case 16: run<16, T>(in, out); return 0;
+        case 18: run<18, T>(in, out); return 0;
+        case 20: run<20, T>(in, out); return 0;
+        case 21: run<21, T>(in, out); return 0;
+        case 24: run<24, T>(in, out); return 0;
+        case 25: run<25, T>(in, out); return 0;
+        case 27: run<27, T>(in, out); return 0;
+        case 28: run<28, T>(in, out); return 0;
+        case 30: run<30, T>(in, out); return 0;
+        case 32: run<32, T>(in, out); return 0;
         default: return 1;
     }
 }

@@ -28,9 +28,15 @@ struct Span {
     }
 };
 
-// The product of the kernel's twiddle rows that gives w^r (rows w, w^2, w^4, w^8).
-cd power(const std::vector<cd>& tw, int64_t off, int ns, int jm, int r) {
+// The product of the kernel's twiddle rows that gives w^r (rows w, w^2, w^4, w^8; above radix 16 w, w^2, w^3
+// and w^4, w^8, w^12, ..).
+cd power(const std::vector<cd>& tw, int64_t off, int ns, int jm, int r, int R = 16) {
     cd w = 1.0;
+    if (R > 16) {
+        if (r % 4) w *= tw[off + int64_t(r % 4 - 1) * ns + jm];
+        if (r / 4) w *= tw[off + int64_t(2 + r / 4) * ns + jm];
+        return w;
+    }
     for (int q = 0; (1 << q) <= r; ++q)
         if (r & (1 << q)) w *= tw[off + int64_t(q) * ns + jm];
     return w;
@@ -99,7 +105,7 @@ void run_smooth(const PlanSpec& plan, const PassSpec& ps, Span& src, Span& dst, 
                     const int jm = last ? j : j % ns;
                     if (jm >= ns) throw std::runtime_error("twiddle index outside its stage");
                     for (int r = 1; r < R; ++r)
-                        if (ns > 1) v[r] *= power(tw, off, ns, jm, r);
+                        if (ns > 1) v[r] *= power(tw, off, ns, jm, r, R);
                     for (int q = 0; q < R; ++q) {
                         u[q] = 0.0;
                         for (int r = 0; r < R; ++r) u[q] += v[r] * cis_neg(int64_t(q) * r, R);

@@ -46,6 +46,22 @@ def test_contiguous(sf, torch, shape, batch, dbl):
         assert rel_l2(o.cpu().numpy(), fp64_fft(x, shape, batch, d, norm_scale(norm, d, n))) <= tol(n, dbl)
 
 
+@pytest.mark.parametrize("shape,batch", [
+    ([324], 1), ([324], 700), ([500], 301), ([1024], 13), ([945], 7), ([2401], 5), ([6000], 3), ([12288], 2), ([291600], 2),
+    ([810, 24], 2), ([1024, 20], 3),
+], ids=str)
+def test_wide_radices(sf, torch, shape, batch):
+    """Radices above 16: two and three stages of a line, columns, both passes of a four-step."""
+    n = int(np.prod(shape))
+    x = uniform_complex(n * batch, n + batch, np.complex64)
+    for d, norm in ((-1, 0), (1, 3)):
+        p = sf.plan_many_dft("float", shape, batch, sf.direction(d), sf.plan_options(normalization=sf.normalization(norm)))
+        a = torch.from_numpy(x).cuda()
+        o = torch.full_like(a, 9.0)
+        p.execute(a, o).synchronize()
+        assert rel_l2(o.cpu().numpy(), fp64_fft(x, shape, batch, d, norm_scale(norm, d, n))) <= tol(n, False)
+
+
 @pytest.mark.parametrize("dbl", [False, True], ids=["float", "double"])
 @pytest.mark.parametrize("n,b,src,dst", [
     (64, 24, (1, 24), (64, 1)), (64, 1, (1, 5), (64, 1)), (60, 7, (1, 9), (1, 11)), (100, 5, (107, 1), (103, 1)),

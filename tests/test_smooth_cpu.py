@@ -25,6 +25,13 @@ def test_composite_butterflies(radix):
     assert np.max(np.abs(butterfly(radix, x, double=False) - np.fft.fft(x))) < 2e-6 * radix
 
 
+@pytest.mark.parametrize("radix", [18, 20, 21, 24, 25, 27, 28, 30, 32])
+def test_wide_butterflies(radix):
+    x = gaussian_complex(radix, radix, np.complex128)
+    assert np.max(np.abs(butterfly(radix, x) - np.fft.fft(x))) < 1e-14 * radix
+    assert np.max(np.abs(butterfly(radix, x, double=False) - np.fft.fft(x))) < 2e-6 * radix
+
+
 def test_catalog_geometry():
     """Ids number the entries; radices multiply to the length; lines fit the block, the registers of an
     SM and its shared memory; the padded row holds the line; mappings with a column side take a power of
@@ -34,7 +41,7 @@ def test_catalog_geometry():
     assert len({(e[1], e[2], e[3], e[4]) for e in entries}) == len(entries)
     for e in entries:
         _, dbl, kind, feat, n, tpl, w, pads, pitch, maxt, minb, *radices = e
-        assert np.prod(radices) == n and len(radices) >= 2 and max(radices) <= 16, e
+        assert np.prod(radices) == n and len(radices) >= 2 and max(radices) <= (16 if dbl else 32), e
         assert (w * tpl + 31) // 32 * 32 == maxt <= 1024 and maxt * minb <= 2048, e
         assert pitch > (n - 1) + ((n - 1) >> pads if pads else 0), e
         assert w * pitch * (16 if dbl else 8) <= 227 * 1024, e
@@ -67,6 +74,17 @@ def test_contiguous_plans_by_thread(shape, batch, double):
         y = smooth_run(x, shape, batch, d, norm, double, ip)
         if y is None:
             pytest.skip("a pass of this plan is not a 7-smooth kernel")
+        assert rel_l2(y, fp64_fft(x, shape, batch, d, norm_scale(norm, d, n))) < 1e-13
+
+
+# radices above 16 in every place: two stages of a line, a column and both passes of a four-step, three stages
+@pytest.mark.parametrize("shape,batch", [([324], 7), ([500], 3), ([1024], 5), ([945], 2), ([6000], 2), ([12288], 1),
+                                         ([810, 24], 1), ([1024, 20], 1), ([291600], 1)], ids=str)
+def test_wide_radices_by_thread(shape, batch):
+    n = int(np.prod(shape))
+    x = gaussian_complex(n * batch, n + batch, np.complex128)
+    for d, norm, ip in ((-1, 3, False), (1, 2, True)):
+        y = smooth_run(x, shape, batch, d, norm, False, ip)
         assert rel_l2(y, fp64_fft(x, shape, batch, d, norm_scale(norm, d, n))) < 1e-13
 
 
