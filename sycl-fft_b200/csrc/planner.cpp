@@ -4,6 +4,7 @@
 #include "fixed_catalog.h"
 #include "fused4_catalog.h"
 #include "piped_catalog.h"
+#include "smooth_piped_catalog.h"
 #include "smooth_catalog.h"
 #include "tc_catalog.h"
 #include "bluestein_catalog.h"
@@ -449,6 +450,11 @@ struct Builder {
         if (!e || static_cast<int64_t>(e->w) * e->pitch * cs > smem_limit) return;
         ps.tables.smooth = smooth_table(*e);
         ps.smooth_id = e->id;
+        const SmoothEntry* q = kind == kSmoothKK && !req.no_piped && p.in.cs % 2 == 0 ? find_smooth_piped(req.dbl, 0, p.n) : nullptr;
+        if (q && (static_cast<int64_t>(q->n) + q->pitch) * cs + 16 <= smem_limit) {
+            ps.tables.spiped = smooth_table(*q);
+            ps.spiped_id = q->id;
+        }
     }
 
     bool fits(int64_t n, int mode) {
@@ -1707,6 +1713,29 @@ const SmoothEntry* find_smooth(bool dbl, int kind, int feat, int n) {
 }
 
 namespace {
+const std::vector<SmoothEntry>& smooth_piped_entries() {
+    static const std::vector<SmoothEntry> all = {
+#define SFB_X(ID, DBL, KIND, FEAT, N, TPL, W, PADS, PITCH, MAXT, MINB, ...) \
+    {ID, DBL, KIND, FEAT, N, TPL, W, PADS, PITCH, MAXT, MINB, {__VA_ARGS__}, count_args(__VA_ARGS__)},
+        SFB_SPIPED_CATALOG(SFB_X)
+#undef SFB_X
+    };
+    return all;
+}
+}  // namespace
+
+const SmoothEntry* find_smooth_piped(bool dbl, int feat, int n) {
+    for (const SmoothEntry& e : smooth_piped_entries())
+        if (!dbl && e.feat == feat && e.n == n) return &e;
+    return nullptr;
+}
+
+const SmoothEntry* smooth_piped_entry(int id) {
+    const auto& all = smooth_piped_entries();
+    return id >= 0 && id < static_cast<int>(all.size()) ? &all[id] : nullptr;
+}
+
+namespace {
 // Per stage the rows W_(ns*R)^(r*jm), jm < ns, r = smooth_tw_power(R, row).
 std::vector<std::complex<double>> stage_rows(const std::vector<int>& radices) {
     std::vector<int64_t> key(radices.begin(), radices.end());
@@ -1902,7 +1931,7 @@ std::string describe_plan(const PlanSpec& plan) {
            << ",\"maxv\":" << ps.kc.maxv << ",\"maxt\":" << ps.kc.maxt << ",\"src\":" << int(ps.src)
            << ",\"dst\":" << int(ps.dst) << ",\"bytes\":" << ps.bytes_moved
            << ",\"store_via_smem\":" << p.store_via_smem << ",\"fixed_id\":" << ps.fixed_id
-           << ",\"piped_id\":" << ps.piped_id << ",\"tc_id\":" << ps.tc_id << ",\"blue_id\":" << ps.blue_id << ",\"tma\":" << (ps.tma ? 1 : 0) << ",\"cluster_id\":" << ps.cluster_id << ",\"cluster_pipe\":" << (ps.cluster_pipe ? 1 : 0) << ",\"cluster\":[" << ps.cl_n1 << "," << ps.cl_n2 << ","
+           << ",\"piped_id\":" << ps.piped_id << ",\"spiped_id\":" << ps.spiped_id << ",\"tc_id\":" << ps.tc_id << ",\"blue_id\":" << ps.blue_id << ",\"tma\":" << (ps.tma ? 1 : 0) << ",\"cluster_id\":" << ps.cluster_id << ",\"cluster_pipe\":" << (ps.cluster_pipe ? 1 : 0) << ",\"cluster\":[" << ps.cl_n1 << "," << ps.cl_n2 << ","
            << ps.cl_p << "],\"rader\":" << (ps.rader ? 1 : 0) << ",\"lean\":" << (ps.lean ? 1 : 0)
            << ",\"smooth_id\":" << ps.smooth_id << ",\"smooth_radices\":[";
         if (const SmoothEntry* e = smooth_entry(ps.smooth_id))

@@ -37,6 +37,7 @@ struct TableIds {
     int cl_base = -1;  // base twiddles of the pipelined cluster kernel's 256-point FFTs
     int perm_in = -1, perm_out = -1;  // Rader permutations (PlanSpec::index_tables)
     int smooth = -1;  // stage twiddles of the smooth_catalog.h kernel
+    int spiped = -1;  // and of the smooth_piped_catalog.h kernel
 };
 
 struct KernelChoice {
@@ -83,6 +84,9 @@ struct PassSpec {
     // size-specialised kernel of the 7-smooth lengths (smooth_catalog.h) that runs this pass in place of
     // the kernel named above, with its own stage sequence (table tables.smooth); -1: none
     int smooth_id = -1;
+    // its copy-engine-pipelined form (smooth_piped_catalog.h), used for more lines than SMs and 16-byte aligned
+    // buffers; -1: none
+    int spiped_id = -1;
     // Bluestein / Rader pass on a conv_catalog.h kernel (blue_id is then past the ids of bluestein_catalog.h;
     // the twiddles are tables.smooth); -1: on the kernel of blue_id
     int conv_id = -1;
@@ -124,6 +128,9 @@ struct SmoothEntry {
     int nstages;
 };
 const SmoothEntry* find_smooth(bool dbl, int kind, int feat, int n);
+// The copy-engine-pipelined kernel of whole float lines (smooth_piped_catalog.h; feat 0 or kSmoothPost), if any.
+const SmoothEntry* find_smooth_piped(bool dbl, int feat, int n);
+const SmoothEntry* smooth_piped_entry(int id);
 // Its stage twiddles: per stage the rows W_(ns*R)^(r*jm), jm < ns, r = smooth_tw_power(R, row).
 std::vector<std::complex<double>> smooth_twiddles(const SmoothEntry& e);
 const SmoothEntry* smooth_entry(int id);

@@ -93,6 +93,9 @@ struct BoundPass {
     const FusedBlueEntry* fusedblue = nullptr;
     const SmoothEntry* smooth = nullptr;  // size-specialised kernel of a 7-smooth length, and its twiddles
     const void* smooth_tw = nullptr;
+    const SmoothEntry* spiped = nullptr;  // its pipelined form
+    const void* spiped_tw = nullptr;
+    long long spiped_polls = kSpinLimit;
     const ConvEntry* conv = nullptr;      // or the conv_catalog.h kernel of a Bluestein / Rader pass
 };
 
@@ -261,6 +264,8 @@ struct DevicePlan {
     void* real_tw = nullptr;        // W_N^k, k = 0..N/2 (then the one-pass kernel's stage twiddles)
     const RealFusedEntry* real_fused = nullptr;  // one-pass kernel for N/2 (real_kernel.cu), or none
     const SmoothEntry* real_smooth = nullptr;    // or the one-pass smooth_catalog.h kernel
+    const SmoothEntry* real_spiped = nullptr;    // and its pipelined form (R2C)
+    int64_t real_spiped_off = 0;                 // complex elements from real_tw to its stage twiddles
     int64_t real_base_off = 0;      // complex elements from real_tw to the stage twiddles
     // Real transforms of rank 2-3: `inner` is the 1D real plan of the last axis over every outer
     // line, `outer` the complex plan over the outer axes (last axis untransformed), md_buf the
@@ -530,7 +535,7 @@ DevicePlan* build_plan(PlanRequest req, int device, uint32_t flags, const std::s
         const TableIds& t = ps.tables;
         const bool own = ps.smooth_id >= 0 || ps.conv_id >= 0;
         for (int id : {own ? -1 : t.tw1, own ? -1 : t.tw2, t.premul, t.pointwise, t.postmul, t.tw4_hi, t.tw4_lo, t.tc_tw,
-                       t.cl_base, t.smooth})
+                       t.cl_base, t.smooth, t.spiped})
             if (id >= 0) read[id] = 1;
     }
     std::vector<size_t> offsets(plan->spec.tables.size()), ioffsets(plan->spec.index_tables.size());
@@ -642,6 +647,8 @@ DevicePlan* build_plan(PlanRequest req, int device, uint32_t flags, const std::s
         bp.tp = to_tc(bp.p, tab(ps.tables.tc_tw), plan->status);
         bp.smooth = smooth_entry(ps.smooth_id);
         bp.smooth_tw = tab(ps.tables.smooth);
+        bp.spiped = smooth_piped_entry(ps.spiped_id);
+        bp.spiped_tw = tab(ps.tables.spiped);
         bp.conv = conv_entry(ps.conv_id);
         plan->passes.push_back(bp);
     }
@@ -794,6 +801,13 @@ DevicePlan* create_real_plan_1d(const syclfft_b200_plan_config_v1& cfg, int kind
     } else if (plan->real_smooth) {
         const auto t = smooth_twiddles(*plan->real_smooth);
         table.insert(table.end(), t.begin(), t.end());
+        if (kind == SYCLFFT_B200_REAL_R2C && !plan->spec.req.no_piped)
+            plan->real_spiped = find_smooth_piped(dbl, kSmoothPost, static_cast<int>(h));
+        if (plan->real_spiped) {
+            plan->real_spiped_off = static_cast<int64_t>(table.size());
+            const auto u = smooth_twiddles(*plan->real_spiped);
+            table.insert(table.end(), u.begin(), u.end());
+        }
     }
     std::vector<unsigned char> tw(table.size() * cs);
     for (size_t k = 0; k < table.size(); ++k) {
@@ -1149,7 +1163,14 @@ void execute_real(DevicePlan* plan, const void* in, void* out, cudaStream_t stre
         p.real_tw = plan->real_tw;
         p.conj_in = p.conj_out = r2c ? 0 : 1;  // C2R: the unnormalized inverse as conj(FFT(conj z))
         p.scale = scale;
-        check(launch_smooth(*plan->real_smooth, p, 1, plan->sms, in, out, stream), "fused real transform");
+        // lines of h complex values, h even: every line starts on a 16-byte boundary when the first does
+        if (plan->real_spiped && lines > plan->sms && reinterpret_cast<uintptr_t>(in) % 16 == 0) {
+            p.tw = static_cast<const unsigned char*>(plan->real_tw) + plan->real_spiped_off * 8;
+            check(launch_smooth_piped(*plan->real_spiped, p, plan->sms, plan->status, plan->inner->wait_polls, in, out, stream),
+                  "fused real transform");
+        } else {
+            check(launch_smooth(*plan->real_smooth, p, 1, plan->sms, in, out, stream), "fused real transform");
+        }
     } else if (plan->real_kind == SYCLFFT_B200_REAL_R2C) {
         execute_plan(plan->inner.get(), in, plan->real_buf, stream, batch, 0, -1);
         check(launch_r2c_post(dbl, plan->real_buf, out, h, lines, plan->real_tw, scale, stream), "R2C post-process");
@@ -1272,8 +1293,12 @@ void launch_bound_pass(DevicePlan* plan, const BoundPass& bp, void* src, void* d
     const PassSpec& ps = bp.spec_ref();
     if (bp.smooth) {
         int64_t n_outer = 1;
-        const SmoothParams sp = to_smooth(bp.p, bp.smooth_tw, &n_outer);
-        check(launch_smooth(*bp.smooth, sp, n_outer, plan->sms, src, dst, stream), "FFT pass launch");
+        SmoothParams sp = to_smooth(bp.p, bp.smooth_tw, &n_outer);
+        if (bp.spiped && aligned && sp.n_cols > plan->sms) {
+            sp.tw = bp.spiped_tw;
+            check(launch_smooth_piped(*bp.spiped, sp, plan->sms, plan->status, bp.spiped_polls, src, dst, stream),
+                  "FFT pipelined pass launch");
+        } else check(launch_smooth(*bp.smooth, sp, n_outer, plan->sms, src, dst, stream), "FFT pass launch");
     } else if (bp.conv) {
         FixedParams fp = bp.fp;
         fp.tw = bp.smooth_tw;
@@ -1378,6 +1403,7 @@ void execute_plan(DevicePlan* plan, const void* in, void* out, cudaStream_t stre
     for (size_t i = 0; i < np; ++i) {
         BoundPass bp = rescale(plan->passes[i], batch, planned);
         bp.pp.wait_polls = plan->wait_polls;
+        bp.spiped_polls = plan->wait_polls;
         bp.tp.wait_polls = plan->wait_polls;
         if (flip || set_scale) apply_override(bp, i == 0, i + 1 == np, flip, scale, set_scale);
         if (bp.fused4 && i + 1 < np && bp.p.n_outer >= 3) {

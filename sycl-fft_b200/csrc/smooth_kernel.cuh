@@ -14,7 +14,7 @@
 //    three. Shared-memory traffic (the load/store pipe was 66 to 78% busy) and barriers fall with every
 //    exchange, and the values in flight per SM rise. [15, 8, 5, 5] -> [25, 10, 12]: 3000 x 16384 178 -> 151
 //    us; 810 x 840 four-step [9, 9, 10] and [15, 4, 14] -> [27, 30] and [30, 28]: 680400 x 64 360 -> 310 us;
-//    1024 columns -> rows [16, 8, 8] -> [32, 32]: 240 -> 209 us. 869 of the 2290 float entries, those that
+//    1024 columns -> rows [16, 8, 8] -> [32, 32]: 240 -> 209 us. 869 of the 1820 float entries, those that
 //    gained at least 1.5%: 1.15x (geometric mean). Packed two-value additions (add.f32x2) in their place
 //    gave nothing: the exchanges, not the arithmetic, fill the time.
 //  * up to 16 values a thread in double too, at 128 registers and half the threads: the same bytes in

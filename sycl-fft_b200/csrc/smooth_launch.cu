@@ -17,6 +17,10 @@ static_assert(SFB_CONV_PARTS == 8, "SFB_EACH_CONV_PART lists the parts");
 #define SFB_DECL(P) const SmoothKernel* smooth_part_##P(int* count);
 SFB_EACH_PART(SFB_DECL)
 #undef SFB_DECL
+#define SFB_EACH_SPIPED_PART(F) F(0) F(1) F(2) F(3)
+#define SFB_DECL(P) const SmoothKernel* smooth_piped_part_##P(int* count);
+SFB_EACH_SPIPED_PART(SFB_DECL)
+#undef SFB_DECL
 #define SFB_DECL(P) const ConvKernel* conv_part_##P(int* count);
 SFB_EACH_CONV_PART(SFB_DECL)
 #undef SFB_DECL
@@ -28,6 +32,18 @@ KernelSet& smooth_kernels() {
         auto* s = new KernelSet;
 #define SFB_ADD(P) s->add(smooth_part_##P);
         SFB_EACH_PART(SFB_ADD)
+#undef SFB_ADD
+        s->finish();
+        return s;
+    }();
+    return *k;
+}
+
+KernelSet& smooth_piped_kernels() {
+    static KernelSet* k = [] {
+        auto* s = new KernelSet;
+#define SFB_ADD(P) s->add(smooth_piped_part_##P);
+        SFB_EACH_SPIPED_PART(SFB_ADD)
 #undef SFB_ADD
         s->finish();
         return s;
@@ -61,6 +77,18 @@ cudaError_t launch_smooth(const SmoothEntry& e, SmoothParams p, int64_t n_outer,
     p.col_tiles = (p.n_cols + p.w - 1) / p.w;
     void* args[] = {&p, const_cast<void**>(&in), &out};
     return smooth_kernels().launch(e.id, n_outer * p.col_tiles, threads, p.w * line, e.w * line, args, stream);
+}
+
+cudaError_t launch_smooth_piped(const SmoothEntry& e, const SmoothParams& p, int sms, int* status, long long wait_polls,
+                                const void* in, void* out, cudaStream_t stream) {
+    SmoothPipedParams q;
+    q.s = p;
+    q.status = status;
+    q.wait_polls = wait_polls;
+    const size_t smem = static_cast<size_t>(smooth_piped_smem(e.n, e.pitch));
+    const int64_t ctas = static_cast<int64_t>(sms) * e.minb;
+    void* args[] = {&q, const_cast<void**>(&in), &out};
+    return smooth_piped_kernels().launch(e.id, p.n_cols < ctas ? p.n_cols : ctas, e.maxt, smem, smem, args, stream);
 }
 
 cudaError_t launch_conv(const ConvEntry& e, FixedParams p, int64_t n_outer, int sms, const void* in, void* out,

@@ -7,6 +7,7 @@
 
 #include "planner.hpp"
 #include "smooth_kernel.cuh"
+#include "smooth_piped.cuh"
 
 namespace sfb {
 
@@ -14,6 +15,11 @@ namespace sfb {
 // the caller, the tile geometry (w, col_tiles) here.
 cudaError_t launch_smooth(const SmoothEntry& e, SmoothParams p, int64_t n_outer, int sms, const void* in, void* out,
                           cudaStream_t stream);
+
+// Runs p.n_cols whole lines on a smooth_piped_catalog.h kernel; buffers and input pitch are multiples of 16
+// bytes. `status` is set to 1 when a copy is not there after `wait_polls` polls.
+cudaError_t launch_smooth_piped(const SmoothEntry& e, const SmoothParams& p, int sms, int* status, long long wait_polls,
+                                const void* in, void* out, cudaStream_t stream);
 
 // One kernel of a compiled part of the catalog.
 struct SmoothKernel {

@@ -120,3 +120,32 @@ def test_real_one_pass(sf, torch, h, batch, dbl):
     back = torch.full((batch * n,), 9.0, dtype=b.real_dtype, device="cuda")
     b.execute(torch.from_numpy(s).cuda(), back).synchronize()
     assert rel_l2(back.cpu().numpy(), x.reshape(-1).astype(np.float64)) <= 2 * tol(n, dbl)
+
+
+# just above one line per SM, several lines per block with a remainder; the shortest and longest entries
+@pytest.mark.parametrize("n,batch", [(4116, 301), (5488, 149), (9000, 1000), (12544, 297), (14400, 150)])
+def test_pipelined_lines(sf, torch, n, batch):
+    """More lines than SMs on the pipelined kernels, out of place, in place and in the other direction; buffers
+    off a 16-byte boundary and a few lines of the same plan on the plain ones."""
+    x = uniform_complex(n * batch, n, np.complex64)
+    for d, norm, in_place in ((-1, 0, False), (1, 3, True)):
+        opts = sf.plan_options(placement=sf.placement.in_place if in_place else sf.placement.out_of_place,
+                               normalization=sf.normalization(norm))
+        p = sf.plan_many_dft("float", [n], batch, sf.direction(d), opts)
+        assert p.describe()["passes"][0]["spiped_id"] >= 0
+        ref = fp64_fft(x, [n], batch, d, norm_scale(norm, d, n))
+        for off in (0, 1):
+            a = torch.zeros(n * batch + 1, dtype=torch.complex64, device="cuda")[off:off + n * batch]
+            a.copy_(torch.from_numpy(x))
+            o = a if in_place else torch.zeros(n * batch + 1, dtype=torch.complex64, device="cuda")[off:off + n * batch]
+            (p.execute(a) if in_place else p.execute(a, o)).synchronize()
+            assert rel_l2(o.cpu().numpy(), ref) <= tol(n, False)
+
+
+@pytest.mark.parametrize("h,batch", [(4116, 149), (12544, 301), (13440, 150)])
+def test_pipelined_real(sf, torch, h, batch):
+    x = np.random.default_rng(h).uniform(-1, 1, (batch, 2 * h)).astype(np.float32)
+    p = sf.plan_dft_r2c_1d("float", 2 * h, batch, sf.plan_options(normalization=sf.normalization(0)))
+    o = torch.full((batch, h + 1), 9.0, dtype=torch.complex64, device="cuda")
+    p.execute(torch.from_numpy(x).cuda(), o).synchronize()
+    assert rel_l2(o.cpu().numpy(), np.fft.rfft(x.astype(np.float64), axis=-1)) <= tol(2 * h, False)

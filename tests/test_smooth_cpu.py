@@ -49,6 +49,22 @@ def test_catalog_geometry():
         assert feat in (0, {KK: 0, CC: 1}.get(kind, 0)) or (kind == KK and feat in (2, 4)), e
 
 
+def test_pipelined_catalog_geometry():
+    """Even float lines, one per block; copy buffer, work buffer and barrier of MINB blocks fit an SM; every
+    entry's length has the plain kernel that misaligned buffers and few lines take."""
+    entries = catalog("smooth_piped_catalog.h")
+    plain = {(e[3], e[4]) for e in catalog() if e[1] == 0 and e[2] == KK}
+    assert sorted(e[0] for e in entries) == list(range(len(entries)))
+    assert len({(e[3], e[4]) for e in entries}) == len(entries)
+    for e in entries:
+        _, dbl, kind, feat, n, tpl, w, pads, pitch, maxt, minb, *radices = e
+        assert dbl == 0 and kind == KK and w == 1 and feat in (0, 2) and n % 2 == 0 and (feat, n) in plain, e
+        assert np.prod(radices) == n and len(radices) >= 2 and max(radices) <= 32, e
+        assert (tpl + 31) // 32 * 32 == maxt <= 1024 and maxt * minb <= 2048, e
+        assert pitch > (n - 1) + ((n - 1) >> pads if pads else 0), e
+        assert minb * ((n + pitch) * 8 + 16 + 1024) <= 228 * 1024 and (n + pitch) * 8 + 16 <= 227 * 1024, e
+
+
 def test_convolution_catalog_geometry():
     entries = catalog("conv_catalog.h")
     assert [e[0] for e in entries] == list(range(len(entries)))
