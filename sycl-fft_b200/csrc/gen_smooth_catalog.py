@@ -13,8 +13,8 @@ first choices are within 10% of the fastest on average and up to 2x off for sing
 committed catalog holds the fastest of 20,000 candidates timed on B200 (128 MB of input each). A
 complex length is left out where the power-of-two kernel of fixed_catalog.h was faster (64-point float
 lines). The real transforms (FEAT 2 and 4) take the layouts chosen for complex lines, or one with a radix
-above 16 where that was faster for them. Radices above 16 (float only: a double butterfly of 18 values takes
-more than 128 registers) are taken where they timed at least 1.5% below the best layout of radices to 16.
+above 16 where that was faster for them. Radices above 16 (float only; the values
+of a double butterfly would take twice the registers) are taken where they timed at least 1.5% below the best layout of radices to 16.
 """
 import itertools
 import math

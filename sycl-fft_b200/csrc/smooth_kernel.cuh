@@ -13,8 +13,8 @@
 //  * float radices to 32 at up to 128 registers a thread: 256 to 1024 points in two stages, longer lines in
 //    three. Shared-memory traffic (the load/store pipe was 66 to 78% busy) and barriers fall with every
 //    exchange, and the values in flight per SM rise. [15, 8, 5, 5] -> [25, 10, 12]: 3000 x 16384 178 -> 151
-//    us; 810 x 840 four-step [9, 9, 10] and [15, 4, 14] -> [27, 30] and [30, 28]: 680400 x 64 360 -> 310 us;
-//    1024 columns -> rows [16, 8, 8] -> [32, 32]: 240 -> 209 us. 869 of the 1820 float entries, those that
+//    to 161 us (several cards); 810 x 840 four-step [9, 9, 10] and [15, 4, 14] -> [27, 30] and [30, 28]: 680400 x 64 360 -> 310 to 326 us;
+//    1024 columns -> rows [16, 8, 8] -> [32, 32]: 240 -> 209 to 224 us. 869 of the 1820 float entries, those that
 //    gained at least 1.5%: 1.15x (geometric mean). Packed two-value additions (add.f32x2) in their place
 //    gave nothing: the exchanges, not the arithmetic, fill the time.
 //  * up to 16 values a thread in double too, at 128 registers and half the threads: the same bytes in
@@ -22,8 +22,8 @@
 //
 // What bounds it: HBM for the lines up to about 2000 points (4.9 to 6.4 of the 6.5 TB/s copy rate), the
 // issue slots and exchanges of the longer ones, one or two blocks of which fill an SM. Times per execute on
-// B200 against the runtime-length kernels: 3000 x 16384 float 337 -> 151 us, 680400 x 64 float (810 x 840
-// four-step) 638 -> 310 us, 840 x 1200 x 4 float 101 -> 34 us; complex<double> 65536 x 512 (256 x 256)
+// B200 against the runtime-length kernels: 3000 x 16384 float 337 -> 161 us, 680400 x 64 float (810 x 840
+// four-step) 638 -> 326 us, 840 x 1200 x 4 float 101 -> 34 us; complex<double> 65536 x 512 (256 x 256)
 // 415 -> 354 us against fixed_kernel.cuh. All 691 whole-line lengths above 15: 1.96x (geometric mean, 64 MB
 // batches), columns 2.3x, four-steps to 2^20 1.67x.
 #pragma once
@@ -94,8 +94,9 @@ __device__ __forceinline__ void smooth_twiddle(C* u, const C* __restrict__ tw, i
 }
 
 // Radices above 16: the power 4h + s is one product of the rows w^(4h) and w^s (s = 1, 2, 3), so that no power
-// is more than one product away from the table and few of them are live beside the values. Against
-// products of w, w^2, w^4, w^8 and w^16 alone: 3000 x 16384 158 -> 151 us, 680400 x 64 323 -> 310 us.
+// is more than one product away from the table and few of them are live beside the values. Over 43 lengths
+// from 324 to 10^6 points the errors against FP64 are 0.9 to 1.04 times those of full tables (products
+// of w, w^2, w^4, w^8 and w^16: 1.6e-7 against 1.4e-7 at one length).
 template <int R, int NS, class C>
 __device__ __forceinline__ void smooth_twiddle_wide(C* u, const C* __restrict__ tw, int jm) {
     const C w1 = __ldg(tw + jm), w2 = __ldg(tw + NS + jm), w3 = __ldg(tw + 2 * NS + jm);
