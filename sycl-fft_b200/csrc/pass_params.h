@@ -32,8 +32,9 @@ enum : int { kModeK = 0, kModeC = 1 };         // thread mapping / coalesced dim
 // (element stride 1), C lanes walk adjacent lines (line stride 1).
 enum : int { kSmoothKK = 0, kSmoothCC = 1, kSmoothCK = 2, kSmoothKC = 3 };
 // Features of a smooth_kernel.cuh instantiation: four-step twiddle on the store; real transforms of length
-// 2N, bins formed after the last stage (R2C) or read before the first (C2R).
-enum : int { kSmoothTw4 = 1, kSmoothPost = 2, kSmoothPre = 4 };
+// 2N, bins formed after the last stage (R2C) or read before the first (C2R); columns whose tiles run on across
+// outer indices (not in the catalog: the second form of its plain column entries, smooth_runs_on).
+enum : int { kSmoothTw4 = 1, kSmoothPost = 2, kSmoothPre = 4, kSmoothRun = 8 };
 // Rows of a radix-R stage's twiddle table in smooth_kernel.cuh: W^(r*jm) for r = 1, 2, 4, 8 below R; above
 // radix 16 for r = 1, 2, 3, 4, 8, 12, .. below R.
 #if defined(__CUDACC__)
@@ -41,6 +42,22 @@ __host__ __device__
 #endif
 constexpr int smooth_tw_entries(int R) { return R > 16 ? 3 + (R - 1) / 4 : R > 8 ? 4 : R > 4 ? 3 : R > 2 ? 2 : 1; }
 inline int smooth_tw_power(int R, int q) { return R <= 16 ? 1 << q : q < 3 ? q + 1 : 4 * (q - 2); }  // of row q
+// Column tiles of smooth_kernel.cuh over arrays narrower than a tile (the first axis of [500, 2]): a tile takes its
+// W lines from several outer indices, line l being column l % cols of outer index l / cols. One tile per outer
+// index leaves W - cols of W lanes idle, which made two columns slower than the runtime-length kernel. 48 MB
+// arrays on B200, runtime-length / one tile per outer index / run on: double 375 x 2 69 / 98 / 57 us, float
+// 175 x 2 170 / 208 / 122 us; geometric means over the 177 lengths of each precision, of the runtime-length
+// kernel's time and of the idle lanes': 2 columns 1.5x and 1.33x, 3 columns 1.5x and 1.16x, 6 columns 1.8x and 1.06x.
+struct RunLine {
+    int64_t o, c;
+};
+#if defined(__CUDACC__)
+__host__ __device__
+#endif
+inline RunLine smooth_run_line(uint32_t l, uint32_t cols) { return {l / cols, l % cols}; }
+inline bool smooth_runs_on(int kind, int feat, int w, int64_t n_cols, int64_t n_outer) {
+    return kind == kSmoothCC && feat == 0 && w > 2 && n_cols < w && n_outer > 1 && n_outer * n_cols <= INT32_MAX;
+}
 enum : int { kSelNone = 0, kSelCol = 1, kSelOuterLo = 2, kSelColMod = 3 };
 
 struct LineLayout {

@@ -41,6 +41,7 @@ struct SmoothParams {
     int64_t n_cols = 1;     // lines per outer index
     int64_t col_tiles = 1;  // ceil(n_cols / w)
     int w = 1;              // lines per CTA (KK; the other mappings use the compile-time W)
+    int run_cols = 0;       // kSmoothRun: columns per outer index; n_cols then counts the lines of all outer indices
     int64_t in_hi = 0, in_cs = 0, in_ks = 1;     // element (o, c, k) at o * hi + c * cs + k * ks
     int64_t out_hi = 0, out_cs = 0, out_ks = 1;  // (K sides: ks = 1; C sides: cs = 1)
     const void* tw = nullptr;  // stage twiddles (smooth_tw_entries)
@@ -349,6 +350,7 @@ __global__ void __launch_bounds__(MAXT, MINB)
     fft_smooth_kernel(const __grid_constant__ SmoothParams P, const cplx<T>* in, cplx<T>* out) {
     using C = cplx<T>;
     static_assert(!(FEAT & (kSmoothPost | kSmoothPre)) || KIND == kSmoothKK, "whole contiguous lines");
+    static_assert(!(FEAT & kSmoothRun) || (KIND == kSmoothCC && FEAT == kSmoothRun), "plain columns");
     extern __shared__ __align__(16) unsigned char smem_raw[];
     SmoothCtx<T> X;
     X.sm = reinterpret_cast<C*>(smem_raw);
@@ -377,8 +379,14 @@ __global__ void __launch_bounds__(MAXT, MINB)
     const int64_t co = (KIND == kSmoothKK ? tile * lines : c0) + X.w_out;
     X.in_ok = X.act_in && ci < P.n_cols;
     X.out_ok = X.act_out && co < P.n_cols;
-    X.gin = in + o * P.in_hi + (CIN ? ci : ci * P.in_cs);
-    X.gout = out + o * P.out_hi + (COUT ? co : co * P.out_cs);
+    if constexpr (FEAT & kSmoothRun) {
+        const RunLine l = smooth_run_line(static_cast<uint32_t>(ci), static_cast<uint32_t>(P.run_cols));
+        X.gin = in + l.o * P.in_hi + l.c;
+        X.gout = out + l.o * P.out_hi + l.c;
+    } else {
+        X.gin = in + o * P.in_hi + (CIN ? ci : ci * P.in_cs);
+        X.gout = out + o * P.out_hi + (COUT ? co : co * P.out_cs);
+    }
     if constexpr (FEAT & kSmoothTw4) {
         X.sel = static_cast<int>(co);
         X.tw4_hi = static_cast<const C*>(P.tw4_hi);

@@ -14,7 +14,7 @@ static_assert(SFB_SMOOTH_PARTS == 24, "SFB_EACH_PART lists the parts");
 #define SFB_EACH_CONV_PART(F) F(0) F(1) F(2) F(3) F(4) F(5) F(6) F(7)
 static_assert(SFB_CONV_PARTS == 8, "SFB_EACH_CONV_PART lists the parts");
 
-#define SFB_DECL(P) const SmoothKernel* smooth_part_##P(int* count);
+#define SFB_DECL(P) const SmoothKernel* smooth_part_##P(int* count); const SmoothKernel* smooth_run_part_##P(int* count);
 SFB_EACH_PART(SFB_DECL)
 #undef SFB_DECL
 #define SFB_EACH_SPIPED_PART(F) F(0) F(1) F(2) F(3)
@@ -31,6 +31,18 @@ KernelSet& smooth_kernels() {
     static KernelSet* k = [] {
         auto* s = new KernelSet;
 #define SFB_ADD(P) s->add(smooth_part_##P);
+        SFB_EACH_PART(SFB_ADD)
+#undef SFB_ADD
+        s->finish();
+        return s;
+    }();
+    return *k;
+}
+
+KernelSet& smooth_run_kernels() {
+    static KernelSet* k = [] {
+        auto* s = new KernelSet;
+#define SFB_ADD(P) s->add(smooth_run_part_##P);
         SFB_EACH_PART(SFB_ADD)
 #undef SFB_ADD
         s->finish();
@@ -74,9 +86,16 @@ cudaError_t launch_smooth(const SmoothEntry& e, SmoothParams p, int64_t n_outer,
         p.w = lines_per_block(e.w, p.n_cols, sms);
         threads = (p.w * e.tpl + 31) / 32 * 32;
     }
+    const bool run = smooth_runs_on(e.kind, e.feat, e.w, p.n_cols, n_outer);
+    if (run) {
+        p.run_cols = static_cast<int>(p.n_cols);
+        p.n_cols *= n_outer;
+        n_outer = 1;
+    }
     p.col_tiles = (p.n_cols + p.w - 1) / p.w;
     void* args[] = {&p, const_cast<void**>(&in), &out};
-    return smooth_kernels().launch(e.id, n_outer * p.col_tiles, threads, p.w * line, e.w * line, args, stream);
+    return (run ? smooth_run_kernels() : smooth_kernels())
+        .launch(e.id, n_outer * p.col_tiles, threads, p.w * line, e.w * line, args, stream);
 }
 
 cudaError_t launch_smooth_piped(const SmoothEntry& e, const SmoothParams& p, int sms, int* status, long long wait_polls,

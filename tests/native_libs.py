@@ -147,3 +147,14 @@ def real_pair(pre, a, c, w, half=0.5):
     out = np.zeros(4)
     L.sfb_check_real_pair(int(pre), float(half), xin.ctypes.data, out.ctypes.data)
     return out[0] + 1j * out[1], out[2] + 1j * out[3]
+
+
+def narrow_lines(kind, feat, w, n_cols, n_outer):
+    """(outer, column) of every line of column tiles that run on across outer indices, in tile order; None
+    where the tiles end with the columns."""
+    L = _load("libnarrow_check.so")
+    L.narrow_lines.restype = ctypes.c_int64
+    L.narrow_lines.argtypes = [ctypes.c_int] * 3 + [ctypes.c_int64] * 2 + [ctypes.c_void_p] * 2
+    o, c = np.zeros(n_cols * n_outer, np.int64), np.zeros(n_cols * n_outer, np.int64)
+    n = L.narrow_lines(kind, feat, w, n_cols, n_outer, o.ctypes.data, c.ctypes.data)
+    return None if n < 0 else (o[:n], c[:n])

@@ -149,3 +149,39 @@ def test_pipelined_real(sf, torch, h, batch):
     o = torch.full((batch, h + 1), 9.0, dtype=torch.complex64, device="cuda")
     p.execute(torch.from_numpy(x).cuda(), o).synchronize()
     assert rel_l2(o.cpu().numpy(), np.fft.rfft(x.astype(np.float64), axis=-1)) <= tol(2 * h, False)
+
+
+@pytest.mark.parametrize("dbl", [False, True], ids=["float", "double"])
+@pytest.mark.parametrize("shape,batch", [
+    ([18, 2], 1), ([18, 2], 9), ([64, 3], 5), ([375, 2], 3), ([448, 2], 4), ([500, 3], 7), ([810, 7], 3), ([1024, 2], 2),
+    ([1029, 3], 3), ([100, 15], 4), ([2048, 2], 5), ([2048, 1], 3), ([20, 30, 2], 3), ([7, 25, 5], 2), ([175, 2], 301),
+], ids=str)
+def test_narrow_arrays(sf, torch, shape, batch, dbl):
+    """Column passes over arrays narrower than a tile, whose tiles run on across outer indices: partial last
+    tiles, in place and out of place, nothing outside the array written, and a smaller batch of the plan."""
+    n = int(np.prod(shape))
+    x = uniform_complex(n * batch, n + batch, np.complex128 if dbl else np.complex64)
+    for d, norm, in_place in ((-1, 0, False), (1, 3, True)):
+        opts = sf.plan_options(placement=sf.placement.in_place if in_place else sf.placement.out_of_place,
+                               normalization=sf.normalization(norm))
+        p = sf.plan_many_dft("double" if dbl else "float", shape, batch, sf.direction(d), opts)
+        a = torch.from_numpy(x).cuda()
+        big = torch.full((n * (batch + 2),), 9.0, dtype=a.dtype, device="cuda")
+        o = big[n:n * (batch + 1)]
+        if in_place:
+            o.copy_(a)
+        (p.execute(o) if in_place else p.execute(a, o)).synchronize()
+        ref = fp64_fft(x, shape, batch, d, norm_scale(norm, d, n))
+        assert rel_l2(o.cpu().numpy(), ref) <= tol(n, dbl)
+        assert torch.all(big[:n] == 9.0) and torch.all(big[n * (batch + 1):] == 9.0)
+        if batch > 1 and not in_place:
+            big.fill_(9.0)
+            import ctypes
+            from syclfft_b200 import _provider
+            err = ctypes.create_string_buffer(_provider.ERR_CAP)
+            rc = p._lib.syclfft_b200_execute_batch(p._handle, a.data_ptr(), big.data_ptr(), batch - 1,
+                                                   torch.cuda.current_stream().cuda_stream, err, _provider.ERR_CAP)
+            assert rc == 0, err.value
+            got = big.cpu().numpy()
+            assert rel_l2(got[:n * (batch - 1)], ref[:n * (batch - 1)]) <= tol(n, dbl)
+            assert np.all(got[n * (batch - 1):] == 9.0)

@@ -8,7 +8,7 @@ import numpy as np
 import pytest
 
 from conftest import fp64_fft, gaussian_complex, norm_scale, rel_l2
-from native_libs import butterfly, describe, real_pair, smooth_run, smooth_run_line
+from native_libs import butterfly, describe, narrow_lines, real_pair, smooth_run, smooth_run_line
 
 KK, CC, CK, KC = 0, 1, 2, 3
 
@@ -190,3 +190,18 @@ def test_real_pairs(n):
         assert abs(a - ref[k]) < 1e-12 and abs(c - ref[n - k]) < 1e-12
         p, q = real_pair(True, ref[k], ref[n - k], w)
         assert abs(p - 2 * z[k]) < 1e-12 and (k == 0 or abs(q - 2 * z[n - k]) < 1e-12)
+
+
+@pytest.mark.parametrize("w", [2, 4, 8, 16])
+def test_narrow_arrays_fill_their_tiles(w):
+    """Column tiles wider than the array take lines of several outer indices: every line once, in memory
+    order; not at and above the tile's width, for one outer index, other mappings or the four-step's columns."""
+    for cols in range(1, 17):
+        for outer in (1, 2, 3, 7, 64, 1001):
+            got = narrow_lines(CC, 0, w, cols, outer)
+            if cols >= w or outer == 1 or w == 2:
+                assert got is None
+                continue
+            assert np.array_equal(got[0] * cols + got[1], np.arange(cols * outer)) and got[1].max() == cols - 1
+        for kind, feat in ((CC, 1), (KK, 0), (CK, 0), (KC, 0)):
+            assert narrow_lines(kind, feat, w, cols, 3) is None
