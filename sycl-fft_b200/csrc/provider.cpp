@@ -12,6 +12,7 @@
 #include <climits>
 #include <cstdlib>
 #include <fstream>
+#include <functional>
 #include <map>
 #include <sstream>
 #include <cstring>
@@ -503,7 +504,7 @@ DevicePlan* create_plan(const syclfft_b200_plan_config_v1& cfg, uint32_t flags, 
     if (device < 0) check(cudaGetDevice(&device), "cudaGetDevice");
     DeviceGuard guard(device);
     std::string tuning;
-    if (cfg.measure && !req.strided_line) {
+    if (cfg.measure) {
         // planning_mode::measure: time the candidate decompositions and kernels
         (void)make_plan(req);  // argument validation before any device work
         req = tune(req, device, &tuning);
@@ -737,8 +738,30 @@ void apply_override(BoundPass& bp, bool first, bool last_pass, bool flip, double
     }
 }
 
-// Real transform of even length N over a complex plan of length N/2 (see real_kernel.cu).
-DevicePlan* create_real_plan_1d(const syclfft_b200_plan_config_v1& cfg, int kind, uint32_t flags) {
+// The tuner times on at most this much memory per buffer: a sub-batch has the same per-line behaviour.
+constexpr uint64_t kTuneBytes = uint64_t(256) << 20;
+
+// planning_mode::measure of a plan that has a one-pass and a multi-pass form: builds each for `batch` transforms
+// with make(one_pass), times them and returns whether the one-pass form is the faster (the tuner's cache keeps it
+// under `key`).
+bool measure_forms(const std::string& key, int device, int64_t batch, uint64_t in_bytes, uint64_t out_bytes,
+                   const std::function<DevicePlan*(bool one_pass)>& make, std::string* report);
+bool measure_real_forms(const syclfft_b200_plan_config_v1& cfg, int kind, uint32_t flags, std::string* report);
+
+// The one-pass kernel of real transforms of length 2h, if there is one and nothing asks for another form.
+const SmoothEntry* real_one_pass(const syclfft_b200_plan_config_v1& cfg, int kind, uint32_t flags, uint64_t h) {
+    const bool dbl = cfg.scalar == SYCLFFT_B200_SCALAR_DOUBLE;
+    const char* fused = std::getenv("SYCLFFT_B200_REAL_FUSED");
+    const char* generic = std::getenv("SYCLFFT_B200_KERNELS");
+    if ((!dbl && (flags & SYCLFFT_B200_CREATE_SPLIT_BF16) != 0) || h > (1u << 20)) return nullptr;
+    if (fused && (std::strcmp(fused, "0") == 0 || std::strcmp(fused, "fixed") == 0)) return nullptr;
+    if (generic && std::strcmp(generic, "generic") == 0) return nullptr;
+    return find_smooth(dbl, kSmoothKK, kind == SYCLFFT_B200_REAL_R2C ? kSmoothPost : kSmoothPre, static_cast<int>(h));
+}
+
+// Real transform of even length N over a complex plan of length N/2 (see real_kernel.cu). planning_mode::measure
+// times the one-pass form against the two passes around the tuned complex plan; `two_pass` asks for the latter.
+DevicePlan* create_real_plan_1d(const syclfft_b200_plan_config_v1& cfg, int kind, uint32_t flags, bool two_pass = false) {
     if (kind != SYCLFFT_B200_REAL_R2C && kind != SYCLFFT_B200_REAL_C2R)
         throw std::invalid_argument("real transform kind must be R2C or C2R");
     if (cfg.rank != 1) throw std::invalid_argument("real transforms are one-dimensional (batched)");
@@ -749,11 +772,19 @@ DevicePlan* create_real_plan_1d(const syclfft_b200_plan_config_v1& cfg, int kind
     if (cfg.direction != dir)
         throw std::invalid_argument(dir < 0 ? "R2C transforms are forward" : "C2R transforms are backward");
     if (cfg.normalization > 3) throw std::invalid_argument("Invalid normalization");
+    const SmoothEntry* smooth = two_pass ? nullptr : real_one_pass(cfg, kind, flags, n / 2);
+    std::string report;
+    if (smooth && cfg.measure && cfg.batch_count > 0 && !measure_real_forms(cfg, kind, flags, &report)) {
+        two_pass = true;
+        smooth = nullptr;
+    }
     syclfft_b200_plan_config_v1 ic = cfg;
     ic.lengths[0] = n / 2;
     ic.in_place = 0;
     ic.normalization = 0;
+    if (smooth) ic.measure = 0;
     std::unique_ptr<DevicePlan> inner(create_plan(ic, flags | SYCLFFT_B200_CREATE_SYNC));
+    if (smooth) inner->spec.tuning = report;
     auto plan = std::make_unique<DevicePlan>();
     plan->device = inner->device;
     plan->sms = inner->sms;
@@ -769,21 +800,15 @@ DevicePlan* create_real_plan_1d(const syclfft_b200_plan_config_v1& cfg, int kind
     const bool dbl = plan->spec.req.dbl;
     const size_t cs = dbl ? 16 : 8;
     const uint64_t h = n / 2;
-    // One pass when N/2 has a smooth_catalog.h kernel with the pre- / post-process (every 7-smooth N/2 that
-    // fits a block; not for split-precision plans, whose inner FFT runs on the tensor cores):
-    // 1.03x to 1.4x the power-of-two kernels of real_kernel.cu and 2.1x (geometric mean over 286 lengths) the
-    // two-pass form. SYCLFFT_B200_REAL_FUSED=0 keeps the two-pass form, =fixed the kernels of real_kernel.cu.
+    // One pass when N/2 has a smooth_catalog.h kernel with the pre- / post-process (not for split-precision
+    // plans, whose inner FFT runs on the tensor cores): 1.03x to 1.4x the power-of-two kernels of real_kernel.cu
+    // and 2.1x (geometric mean over 286 lengths) the two-pass form. SYCLFFT_B200_REAL_FUSED=0 keeps the two-pass
+    // form, =fixed the kernels of real_kernel.cu.
     const char* fused_env = std::getenv("SYCLFFT_B200_REAL_FUSED");
-    const char* generic = std::getenv("SYCLFFT_B200_KERNELS");
     const bool split = !dbl && (flags & SYCLFFT_B200_CREATE_SPLIT_BF16) != 0;
-    if (!split && !(fused_env && std::strcmp(fused_env, "0") == 0)) {
-        const bool take = !(fused_env && std::strcmp(fused_env, "fixed") == 0) &&
-                          !(generic && std::strcmp(generic, "generic") == 0) && h <= (1u << 20);
-        if (take)
-            plan->real_smooth = find_smooth(dbl, kSmoothKK, kind == SYCLFFT_B200_REAL_R2C ? kSmoothPost : kSmoothPre,
-                                            static_cast<int>(h));
-        if (!plan->real_smooth) plan->real_fused = find_real_fused(dbl, static_cast<int64_t>(h));
-    }
+    plan->real_smooth = smooth;
+    if (!smooth && !two_pass && !split && !(fused_env && std::strcmp(fused_env, "0") == 0))
+        plan->real_fused = find_real_fused(dbl, static_cast<int64_t>(h));
     const bool one_pass = plan->real_fused || plan->real_smooth;
     plan->spec.scratch_elements = one_pass ? 0 : inner->spec.scratch_elements + h * cfg.batch_count;
     DeviceGuard guard(plan->device);
@@ -827,6 +852,23 @@ DevicePlan* create_real_plan_1d(const syclfft_b200_plan_config_v1& cfg, int kind
     check(cudaEventCreateWithFlags(&plan->done, cudaEventDisableTiming), "cudaEventCreate");
     plan->inner = std::move(inner);
     return plan.release();
+}
+
+bool measure_real_forms(const syclfft_b200_plan_config_v1& cfg, int kind, uint32_t flags, std::string* report) {
+    const bool dbl = cfg.scalar == SYCLFFT_B200_SCALAR_DOUBLE;
+    const uint64_t n = cfg.lengths[0], cs = dbl ? 16 : 8;
+    syclfft_b200_plan_config_v1 c = cfg;
+    c.batch_count = std::max<uint64_t>(1, std::min<uint64_t>(cfg.batch_count, kTuneBytes / ((n / 2 + 1) * cs)));
+    const std::string key = std::string("|") + (dbl ? "z" : "c") + (kind == SYCLFFT_B200_REAL_R2C ? "|r2c|b" : "|c2r|b") +
+                            std::to_string(c.batch_count) + "|" + std::to_string(n);
+    const uint64_t bytes = c.batch_count * (n / 2 + 1) * cs;
+    return measure_forms(key, cfg.device, static_cast<int64_t>(c.batch_count), bytes, bytes,
+                         [&](bool one_pass) {
+                             syclfft_b200_plan_config_v1 t = c;
+                             t.measure = one_pass ? 0 : 1;
+                             return create_real_plan_1d(t, kind, flags, !one_pass);
+                         },
+                         report);
 }
 
 // Real transforms of rank 1-3 over the last axis (even length N): R2C is the 1D real plan of the
@@ -963,6 +1005,100 @@ void check_layout(const Layout& l, bool output) {
     }
 }
 
+LineLayout line_of(const Layout& l) {
+    LineLayout r;
+    r.cs = l.dist;
+    r.ks = l.len[0] > 1 ? l.stride[0] : 1;
+    return r;
+}
+
+// One-dimensional strided plan whose single pass reads and writes the layouts itself.
+DevicePlan* create_direct_plan(const syclfft_b200_plan_config_v1& cfg, const Layout& in, const Layout& out,
+                               uint32_t flags, const std::string& tuning) {
+    syclfft_b200_plan_config_v1 c = cfg;
+    c.measure = 0;
+    const LineLayout li = line_of(in), lo = line_of(out);
+    std::unique_ptr<DevicePlan> inner(create_plan(c, flags | SYCLFFT_B200_CREATE_SYNC, 0, &li, &lo));
+    inner->spec.tuning = tuning;
+    auto plan = std::make_unique<DevicePlan>();
+    plan->device = inner->device;
+    plan->sms = inner->sms;
+    plan->spec.req = inner->spec.req;
+    plan->spec.transform_size = inner->spec.transform_size;
+    plan->spec.elements = inner->spec.elements;
+    plan->status = inner->status;
+    plan->strided = true;
+    plan->direct = true;
+    plan->in_layout = in;
+    plan->out_layout = out;
+    plan->in_contig = layout_contiguous(in);
+    plan->out_contig = layout_contiguous(out);
+    DeviceGuard guard(plan->device);
+    check(cudaEventCreateWithFlags(&plan->done, cudaEventDisableTiming), "cudaEventCreate");
+    plan->inner = std::move(inner);
+    return plan.release();
+}
+
+// Strided plan as the contiguous plan with a gather and / or a scatter pass around it.
+DevicePlan* create_gather_plan(const syclfft_b200_plan_config_v1& cfg, const Layout& in, const Layout& out,
+                               uint32_t flags) {
+    const bool ic = layout_contiguous(in), oc = layout_contiguous(out);
+    syclfft_b200_plan_config_v1 c = cfg;
+    c.in_place = (!ic && !oc) ? 1 : 0;  // both strided: transform the gathered copy in place
+    std::unique_ptr<DevicePlan> inner(create_plan(c, flags | SYCLFFT_B200_CREATE_SYNC));
+    auto plan = std::make_unique<DevicePlan>();
+    plan->device = inner->device;
+    plan->sms = inner->sms;
+    plan->spec.req = inner->spec.req;
+    plan->spec.req.in_place = cfg.in_place != 0;
+    plan->spec.transform_size = inner->spec.transform_size;
+    plan->spec.elements = inner->spec.elements;
+    plan->status = inner->status;
+    plan->strided = true;
+    plan->in_layout = in;
+    plan->out_layout = out;
+    plan->in_contig = ic;
+    plan->out_contig = oc;
+    const size_t cs = plan->spec.req.dbl ? 16 : 8;
+    plan->spec.scratch_elements = inner->spec.scratch_elements + inner->spec.elements;
+    DeviceGuard guard(plan->device);
+    cudaStream_t ms = memory_stream(plan->device);
+    check(cudaMallocAsync(&plan->pack_buf, inner->spec.elements * cs, ms), "cudaMallocAsync(layout scratch)");
+    check(cudaStreamSynchronize(ms), "layout scratch");
+    check(cudaEventCreateWithFlags(&plan->done, cudaEventDisableTiming), "cudaEventCreate");
+    plan->inner = std::move(inner);
+    return plan.release();
+}
+
+
+// planning_mode::measure of a one-dimensional strided plan: true when the one-pass form is the faster. Timed
+// on dense lines or columns of the same mapping where a side's span exceeds the tuner's 256 MB.
+bool measure_layout_forms(const syclfft_b200_plan_config_v1& cfg, const Layout& in, const Layout& out, uint32_t flags,
+                          std::string* report) {
+    const uint64_t cs = cfg.scalar == SYCLFFT_B200_SCALAR_DOUBLE ? 16 : 8;
+    Layout a = in, b = out;
+    auto span = [](const Layout& l) { return (l.len[0] - 1) * l.stride[0] + (l.batch - 1) * l.dist + 1; };
+    syclfft_b200_plan_config_v1 c = cfg;
+    if (static_cast<uint64_t>(std::max(span(a), span(b))) * cs > kTuneBytes) {
+        c.batch_count = std::max<uint64_t>(1, std::min<uint64_t>(cfg.batch_count, kTuneBytes / (cfg.lengths[0] * cs)));
+        for (Layout* l : {&a, &b}) {
+            l->batch = static_cast<int64_t>(c.batch_count);
+            const bool lines = line_of(*l).ks == 1;
+            l->stride[0] = lines ? 1 : l->batch;
+            l->dist = lines ? l->len[0] : 1;
+        }
+    }
+    std::ostringstream key;
+    key << "|" << (cs == 16 ? "z" : "c") << "|" << (cfg.in_place ? "ip" : "oop") << "|b" << c.batch_count << "|" << cfg.lengths[0]
+        << "|layout";
+    for (const Layout* l : {&a, &b}) key << "|" << l->stride[0] << "," << l->dist;
+    return measure_forms(key.str(), cfg.device, static_cast<int64_t>(c.batch_count), span(a) * cs, span(b) * cs,
+                         [&](bool one_pass) {
+                             return one_pass ? create_direct_plan(c, a, b, flags, "") : create_gather_plan(c, a, b, flags);
+                         },
+                         report);
+}
+
 DevicePlan* create_strided_plan(const syclfft_b200_plan_config_v1& cfg, const syclfft_b200_layout_v1& lay,
                                 uint32_t flags) {
     if (cfg.rank == 0 || cfg.rank > 3) throw std::invalid_argument("FFT rank must be between 1 and 3");
@@ -1011,66 +1147,22 @@ DevicePlan* create_strided_plan(const syclfft_b200_plan_config_v1& cfg, const sy
     if (cfg.rank == 1) {
         // Lines whose sides are each contiguous lines or adjacent columns: where the length has a
         // smooth_catalog.h kernel of those mappings it reads and writes the layouts itself, one HBM pass
-        // instead of two or three (1024 points x 65536, float, columns -> rows: 397 -> 239 us;
-        // 177 lengths of 64 MB matrices 2.4 to 2.7x).
-        LineLayout li, lo;
-        li.cs = in.dist;
-        li.ks = in.len[0] > 1 ? in.stride[0] : 1;
-        lo.cs = out.dist;
-        lo.ks = out.len[0] > 1 ? out.stride[0] : 1;
+        // instead of two or three (1024 points x 65536, float, columns -> rows: 397 -> 224 us;
+        // 177 lengths of 64 MB matrices 2.4 to 2.7x). planning_mode::measure times both forms.
+        const LineLayout li = line_of(in), lo = line_of(out);
         const bool dbl = cfg.scalar == SYCLFFT_B200_SCALAR_DOUBLE;
         const bool split = !dbl && (flags & SYCLFFT_B200_CREATE_SPLIT_BF16) != 0;
         const char* generic = std::getenv("SYCLFFT_B200_KERNELS");
         const int kind = strided_line_kind(li, lo);
         if (kind >= 0 && !split && !(generic && std::strcmp(generic, "generic") == 0) && cfg.lengths[0] <= (1u << 20) &&
             find_smooth(dbl, kind, 0, static_cast<int>(cfg.lengths[0]))) {
-            std::unique_ptr<DevicePlan> inner(create_plan(cfg, flags | SYCLFFT_B200_CREATE_SYNC, 0, &li, &lo));
-            auto plan = std::make_unique<DevicePlan>();
-            plan->device = inner->device;
-            plan->sms = inner->sms;
-            plan->spec.req = inner->spec.req;
-            plan->spec.transform_size = inner->spec.transform_size;
-            plan->spec.elements = inner->spec.elements;
-            plan->status = inner->status;
-            plan->strided = true;
-            plan->direct = true;
-            plan->in_layout = in;
-            plan->out_layout = out;
-            plan->in_contig = ic;
-            plan->out_contig = oc;
-            DeviceGuard guard(plan->device);
-            check(cudaEventCreateWithFlags(&plan->done, cudaEventDisableTiming), "cudaEventCreate");
-            plan->inner = std::move(inner);
-            return plan.release();
+            std::string report;
+            if (!cfg.measure || measure_layout_forms(cfg, in, out, flags, &report))
+                return create_direct_plan(cfg, in, out, flags, report);
         }
     }
-    syclfft_b200_plan_config_v1 c = cfg;
-    c.in_place = (!ic && !oc) ? 1 : 0;  // both strided: transform the gathered copy in place
-    std::unique_ptr<DevicePlan> inner(create_plan(c, flags | SYCLFFT_B200_CREATE_SYNC));
-    auto plan = std::make_unique<DevicePlan>();
-    plan->device = inner->device;
-    plan->sms = inner->sms;
-    plan->spec.req = inner->spec.req;
-    plan->spec.req.in_place = cfg.in_place != 0;
-    plan->spec.transform_size = inner->spec.transform_size;
-    plan->spec.elements = inner->spec.elements;
-    plan->status = inner->status;
-    plan->strided = true;
-    plan->in_layout = in;
-    plan->out_layout = out;
-    plan->in_contig = ic;
-    plan->out_contig = oc;
-    const size_t cs = plan->spec.req.dbl ? 16 : 8;
-    plan->spec.scratch_elements = inner->spec.scratch_elements + inner->spec.elements;
-    DeviceGuard guard(plan->device);
-    cudaStream_t ms = memory_stream(plan->device);
-    check(cudaMallocAsync(&plan->pack_buf, inner->spec.elements * cs, ms), "cudaMallocAsync(layout scratch)");
-    check(cudaStreamSynchronize(ms), "layout scratch");
-    check(cudaEventCreateWithFlags(&plan->done, cudaEventDisableTiming), "cudaEventCreate");
-    plan->inner = std::move(inner);
-    return plan.release();
+    return create_gather_plan(cfg, in, out, flags);
 }
-
 void execute_strided(DevicePlan* plan, const void* in, void* out, cudaStream_t stream, uint64_t batch, int direction,
                      int normalization) {
     const uint64_t planned = plan->spec.req.batch;
@@ -1687,6 +1779,78 @@ PlanRequest apply(PlanRequest r, const Knobs& k) {
     return r;
 }
 
+// One tuner at a time in the process: the cache is shared, and concurrent timings would measure each other.
+// Recursive: the multi-pass form that measure_forms times tunes its inner plan.
+std::recursive_mutex& tune_mutex() {
+    static std::recursive_mutex mu;
+    return mu;
+}
+
+void keep_choice(const std::string& key, const std::string& choice) {
+    tune_cache()[key] = choice;
+    if (const char* path = std::getenv("SYCLFFT_B200_TUNE_CACHE")) {
+        std::ofstream out(path, std::ios::app);
+        out << key << '\t' << choice << '\n';
+    }
+}
+
+// Two timing buffers (the first zeroed) and the private stream they live on, stream-ordered (cudaMallocAsync,
+// cudaFreeAsync): a tuning plan made inside a busy process waits for its own work, not for the device.
+struct TuneBuffers {
+    cudaStream_t stream = nullptr;
+    void *a = nullptr, *b = nullptr;
+    TuneBuffers(uint64_t a_bytes, uint64_t b_bytes) {
+        check(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking), "cudaStreamCreate(autotune)");
+        cudaError_t e = cudaMallocAsync(&a, a_bytes, stream);
+        if (e == cudaSuccess) e = cudaMallocAsync(&b, b_bytes, stream);
+        if (e == cudaSuccess) e = cudaMemsetAsync(a, 0, a_bytes, stream);
+        if (e != cudaSuccess) {
+            release();
+            throw std::runtime_error(std::string("autotune buffers: ") + cudaGetErrorString(e));
+        }
+    }
+    ~TuneBuffers() { release(); }
+    void release() {
+        if (!stream) return;
+        if (a) cudaFreeAsync(a, stream);
+        if (b) cudaFreeAsync(b, stream);
+        cudaStreamSynchronize(stream);
+        cudaStreamDestroy(stream);
+        stream = nullptr;
+    }
+    TuneBuffers(const TuneBuffers&) = delete;
+    TuneBuffers& operator=(const TuneBuffers&) = delete;
+};
+
+bool measure_forms(const std::string& key_tail, int device, int64_t batch, uint64_t in_bytes, uint64_t out_bytes,
+                   const std::function<DevicePlan*(bool one_pass)>& make, std::string* report) {
+    std::lock_guard<std::recursive_mutex> tune_lock(tune_mutex());
+    if (device < 0) check(cudaGetDevice(&device), "cudaGetDevice");
+    DeviceGuard guard(device);
+    cudaDeviceProp prop{};
+    check(cudaGetDeviceProperties(&prop, device), "cudaGetDeviceProperties");
+    const std::string key = prop.name + key_tail;
+    const char* const names[2] = {"multi_pass", "one_pass"};
+    const auto hit = tune_cache().find(key);
+    if (hit != tune_cache().end() && (hit->second == names[0] || hit->second == names[1])) {
+        *report = "{\"choice\":\"" + hit->second + "\",\"cached\":true}";
+        return hit->second == names[1];
+    }
+    TuneBuffers buf(in_bytes, out_bytes);
+    float ms[2];
+    for (int one = 1; one >= 0; --one) {
+        std::unique_ptr<DevicePlan> p(make(one != 0));
+        ms[one] = time_candidate(p.get(), batch, buf.a, buf.b, buf.stream);
+    }
+    const bool one_pass = ms[1] <= ms[0];
+    std::ostringstream rep;
+    rep << "{\"timed_batch\":" << batch << ",\"candidates\":{\"one_pass\":" << ms[1] << ",\"multi_pass\":" << ms[0]
+        << "},\"choice\":\"" << names[one_pass] << "\"}";
+    *report = rep.str();
+    keep_choice(key, names[one_pass]);
+    return one_pass;
+}
+
 PlanRequest tune(const PlanRequest& req, int device, std::string* report) {
     static const Knobs kCandidates[] = {
         {"default", false, false, false, 0, 0, 0, false},    {"generic", true, false, false, 0, 0, 0, false},
@@ -1698,10 +1862,7 @@ PlanRequest tune(const PlanRequest& req, int device, std::string* report) {
         {"split256", false, false, false, 0, 0, 0, false, 256}, {"split512", false, false, false, 0, 0, 0, false, 512},
         {"split1024", false, false, false, 0, 0, 0, false, 1024},
     };
-    // one tuner at a time in the process: the cache is shared, and concurrent timings would
-    // measure each other
-    static std::mutex tune_mu;
-    std::lock_guard<std::mutex> tune_lock(tune_mu);
+    std::lock_guard<std::recursive_mutex> tune_lock(tune_mutex());
     const std::string key = tune_key(req, device);
     auto& cache = tune_cache();
     auto hit = cache.find(key);
@@ -1715,23 +1876,8 @@ PlanRequest tune(const PlanRequest& req, int device, std::string* report) {
     const size_t cs = req.dbl ? 16 : 8;
     const uint64_t elements = checked_element_count(req.shape, req.batch);
     const uint64_t per = elements / req.batch;
-    // time on at most ~256 MB per buffer: a sub-batch has the same per-line kernel behaviour
-    const int64_t batch = static_cast<int64_t>(std::max<uint64_t>(1, std::min<uint64_t>(req.batch, (uint64_t(256) << 20) / (per * cs))));
-    // Everything runs on a private stream, stream-ordered (cudaMallocAsync, cudaFreeAsync): a
-    // tuning plan made inside a busy process waits for its own work, not for the device.
-    cudaStream_t ts = nullptr;
-    check(cudaStreamCreateWithFlags(&ts, cudaStreamNonBlocking), "cudaStreamCreate(autotune)");
-    void *a = nullptr, *b = nullptr;
-    cudaError_t ae = cudaMallocAsync(&a, batch * per * cs, ts);
-    if (ae == cudaSuccess) ae = cudaMallocAsync(&b, batch * per * cs, ts);
-    if (ae == cudaSuccess) ae = cudaMemsetAsync(a, 0, batch * per * cs, ts);
-    if (ae != cudaSuccess) {
-        if (a) cudaFreeAsync(a, ts);
-        if (b) cudaFreeAsync(b, ts);
-        cudaStreamSynchronize(ts);
-        cudaStreamDestroy(ts);
-        throw std::runtime_error(std::string("autotune buffers: ") + cudaGetErrorString(ae));
-    }
+    const int64_t batch = static_cast<int64_t>(std::max<uint64_t>(1, std::min<uint64_t>(req.batch, kTuneBytes / (per * cs))));
+    TuneBuffers buf(batch * per * cs, batch * per * cs);
     std::ostringstream rep;
     rep << "{\"timed_batch\":" << batch << ",\"candidates\":{";
     std::string best_name = "default";
@@ -1756,7 +1902,7 @@ PlanRequest tune(const PlanRequest& req, int device, std::string* report) {
         } catch (...) {
             continue;
         }
-        const float ms = time_candidate(p.get(), batch, a, b, ts);
+        const float ms = time_candidate(p.get(), batch, buf.a, buf.b, buf.stream);
         rep << (first ? "" : ",") << "\"" << k.name << "\":" << ms;
         first = false;
         if (ms < best) {
@@ -1764,17 +1910,9 @@ PlanRequest tune(const PlanRequest& req, int device, std::string* report) {
             best_name = k.name;
         }
     }
-    cudaFreeAsync(a, ts);
-    cudaFreeAsync(b, ts);
-    cudaStreamSynchronize(ts);
-    cudaStreamDestroy(ts);
     rep << "},\"choice\":\"" << best_name << "\"}";
     *report = rep.str();
-    cache[key] = best_name;
-    if (const char* path = std::getenv("SYCLFFT_B200_TUNE_CACHE")) {
-        std::ofstream out(path, std::ios::app);
-        out << key << '\t' << best_name << '\n';
-    }
+    keep_choice(key, best_name);
     for (const auto& k : kCandidates)
         if (best_name == k.name) return apply(req, k);
     return req;
