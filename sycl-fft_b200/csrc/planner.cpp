@@ -14,7 +14,7 @@
 #include <algorithm>
 #include <array>
 #include <cmath>
-#include <initializer_list>
+#include <functional>
 #include <limits>
 #include <map>
 #include <memory>
@@ -96,8 +96,10 @@ int maxt_for(int threads) {
 std::mutex g_table_mu;
 std::map<std::vector<int64_t>, std::shared_ptr<const std::vector<std::complex<double>>>> g_tables;
 
+using TablePtr = std::shared_ptr<const std::vector<std::complex<double>>>;
+
 template <class Make>
-std::shared_ptr<const std::vector<std::complex<double>>> cached_table(std::vector<int64_t> key, Make make) {
+TablePtr cached_table(std::vector<int64_t> key, Make make) {
     {
         std::lock_guard<std::mutex> lock(g_table_mu);
         auto it = g_tables.find(key);
@@ -108,6 +110,68 @@ std::shared_ptr<const std::vector<std::complex<double>>> cached_table(std::vecto
     if (g_tables.size() > 4096) g_tables.clear();  // bound the cache
     g_tables[key] = t;
     return t;
+}
+
+// Per stage the rows W_(ns*R)^(r*jm), jm < ns, r = smooth_tw_power(R, row).
+TablePtr stage_rows(const std::vector<int>& radices) {
+    std::vector<int64_t> key(radices.begin(), radices.end());
+    key.push_back(-600);
+    return cached_table(key, [&] {
+        std::vector<std::complex<double>> t;
+        int64_t ns = 1;
+        for (int R : radices) {
+            for (int q = 0; q < smooth_tw_entries(R); ++q)
+                for (int64_t jm = 0; jm < ns; ++jm) t.push_back(cis_neg(smooth_tw_power(R, q) * jm, ns * R));
+            ns *= R;
+        }
+        return t;
+    });
+}
+
+// A Bluestein or Rader kernel the planner may take: its time per point of the convolution (conv_catalog.h; the
+// entries of bluestein_catalog.h count 1, so that the points alone decide), its shared memory where the entry's
+// own rows decide it, and for forward columns the inverse columns of the same length.
+struct ConvChoice {
+    BlueEntry e;
+    double cost = 1.0;
+    int64_t smem = 0;
+    const ConvChoice* inverse = nullptr;
+};
+// By kind, in catalog order.
+struct ConvChoices {
+    std::vector<ConvChoice> kind[4];
+};
+
+ConvChoices make_conv_choices(bool dbl, bool rader, bool bluestein_catalog) {
+    ConvChoices out;
+    int count = 0;
+    const BlueEntry* old = blue_entries(&count);
+    if (bluestein_catalog) {
+        for (int i = 0; i < count; ++i)
+            if (old[i].dbl == (dbl ? 1 : 0)) out.kind[old[i].kind].push_back({old[i]});
+    } else {
+        for (int i = 0; const ConvEntry* c = conv_entry(i); ++i) {
+            if (c->dbl != (dbl ? 1 : 0) || (c->rader != 0) != rader) continue;
+            BlueEntry e{count + c->id, c->dbl, c->kind, c->n, c->tpl, c->w, c->maxt, {}, c->nstages};
+            std::copy(c->radices, c->radices + c->nstages, e.radices);
+            out.kind[c->kind].push_back({e, static_cast<double>(c->cost), static_cast<int64_t>(c->w) * c->pitch * (dbl ? 16 : 8)});
+        }
+    }
+    for (ConvChoice& f : out.kind[kBlueColsFwd])
+        for (auto i = out.kind[kBlueColsInv].rbegin(); i != out.kind[kBlueColsInv].rend(); ++i)
+            if (i->e.n == f.e.n) f.inverse = &*i;
+    return out;
+}
+
+// Made once: the choice of a convolution length is then a walk over the forward columns and the rows (building and
+// searching the lists on each call took 70 to 300 of a prime length's plan creation, in us on the host).
+const ConvChoices& conv_choice_table(bool dbl, bool rader, bool bluestein_catalog) {
+    static const std::vector<ConvChoices> all = [] {
+        std::vector<ConvChoices> t;
+        for (int i = 0; i < 8; ++i) t.push_back(make_conv_choices(i & 1, i & 2, i & 4));
+        return t;
+    }();
+    return all[(dbl ? 1 : 0) + (rader ? 2 : 0) + (bluestein_catalog ? 4 : 0)];
 }
 
 struct Builder {
@@ -121,6 +185,30 @@ struct Builder {
         plan.table_sizes.push_back(t.size());
         plan.tables.push_back(std::move(t));
         return static_cast<int>(plan.tables.size()) - 1;
+    }
+
+    // A table of n entries that finish_tables makes, if a kernel turns out to read it.
+    std::map<int, std::function<TablePtr()>> pending;
+    int add_pending(size_t n, std::function<TablePtr()> make) {
+        plan.table_sizes.push_back(n);
+        plan.tables.emplace_back();
+        const int id = static_cast<int>(plan.tables.size()) - 1;
+        pending[id] = std::move(make);
+        return id;
+    }
+
+    void finish_tables() {
+        plan.table_read.assign(plan.tables.size(), req.fused_passes ? 1 : 0);
+        for (const PassSpec& ps : plan.passes) {
+            const TableIds& t = ps.tables;
+            const bool own = ps.smooth_id >= 0 || ps.conv_id >= 0;
+            for (int id : {own ? -1 : t.tw1, own ? -1 : t.tw2, t.premul, t.pointwise, t.postmul, t.tw4_hi, t.tw4_lo, t.tc_tw,
+                           t.cl_base, t.smooth, t.spiped})
+                if (id >= 0) plan.table_read[id] = 1;
+        }
+        if (req.tables == TableChoice::none) return;
+        for (auto& [id, make] : pending)
+            if (req.tables == TableChoice::all || plan.table_read[id]) plan.tables[id] = *make();
     }
 
     int add_index_table(std::vector<int32_t> t) {
@@ -156,23 +244,25 @@ struct Builder {
             *table_id = it->second;
             return s;
         }
-        std::vector<int64_t> ckey(radices.begin(), radices.end());
-        ckey.push_back(-100);
         const StageSeq sc = s;
-        auto tw = cached_table(ckey, [&] {
-            std::vector<std::complex<double>> t(std::max(off, 1));
-            int ns2 = 1;
-            for (int i = 0; i < sc.nstages; ++i) {
-                const int R = radices[i];
-                for (int jm = 0; jm < ns2; ++jm)
-                    for (int r = 1; r < R; ++r)
-                        t[sc.tw_off[i] + jm * (R - 1) + (r - 1)] =
-                            cis_neg(static_cast<int64_t>(r) * jm, static_cast<int64_t>(ns2) * R);
-                ns2 *= R;
-            }
-            return t;
+        const size_t entries = static_cast<size_t>(std::max(off, 1));
+        *table_id = add_pending(entries, [sc, radices, entries] {
+            std::vector<int64_t> ckey(radices.begin(), radices.end());
+            ckey.push_back(-100);
+            return cached_table(ckey, [&] {
+                std::vector<std::complex<double>> t(entries);
+                int ns2 = 1;
+                for (int i = 0; i < sc.nstages; ++i) {
+                    const int R = radices[i];
+                    for (int jm = 0; jm < ns2; ++jm)
+                        for (int r = 1; r < R; ++r)
+                            t[sc.tw_off[i] + jm * (R - 1) + (r - 1)] =
+                                cis_neg(static_cast<int64_t>(r) * jm, static_cast<int64_t>(ns2) * R);
+                    ns2 *= R;
+                }
+                return t;
+            });
         });
-        *table_id = add_table(*tw);
         seq_tables[key] = *table_id;
         return s;
     }
@@ -183,19 +273,25 @@ struct Builder {
         key.push_back(-1);  // distinct from the full-table key
         auto it = seq_tables.find(key);
         if (it != seq_tables.end()) return it->second;
-        std::vector<int64_t> ckey(radices.begin(), radices.end());
-        ckey.push_back(-200);
-        auto tw = cached_table(ckey, [&] {
-            std::vector<std::complex<double>> t;
-            int64_t ns = 1;
-            for (int R : radices) {
-                for (int64_t jm = 0; jm < ns; ++jm) t.push_back(cis_neg(jm, ns * R));
-                ns *= R;
-            }
-            if (t.empty()) t.push_back(1.0);
-            return t;
+        size_t entries = 0, reach = 1;
+        for (int R : radices) {
+            entries += reach;
+            reach *= static_cast<size_t>(R);
+        }
+        const int id = add_pending(std::max<size_t>(entries, 1), [radices] {
+            std::vector<int64_t> ckey(radices.begin(), radices.end());
+            ckey.push_back(-200);
+            return cached_table(ckey, [&] {
+                std::vector<std::complex<double>> t;
+                int64_t ns = 1;
+                for (int R : radices) {
+                    for (int64_t jm = 0; jm < ns; ++jm) t.push_back(cis_neg(jm, ns * R));
+                    ns *= R;
+                }
+                if (t.empty()) t.push_back(1.0);
+                return t;
+            });
         });
-        const int id = add_table(*tw);
         seq_tables[key] = id;
         return id;
     }
@@ -407,13 +503,34 @@ struct Builder {
         use_base_table(ps);
     }
 
+    // The rows of stage_rows over the radices; `pair`: then over their reverse (conv_twiddles).
+    int stage_row_table(const std::vector<int>& radices, bool pair) {
+        size_t entries = 0, ns = 1;
+        auto add = [&](int R) {
+            entries += ns * static_cast<size_t>(smooth_tw_entries(R));
+            ns *= static_cast<size_t>(R);
+        };
+        for (int R : radices) add(R);
+        ns = 1;
+        if (pair)
+            for (auto R = radices.rbegin(); R != radices.rend(); ++R) add(*R);
+        return add_pending(entries, [radices, pair]() -> TablePtr {
+            TablePtr t = stage_rows(radices);
+            if (!pair) return t;
+            std::vector<std::complex<double>> both = *t;
+            const TablePtr back = stage_rows(std::vector<int>(radices.rbegin(), radices.rend()));
+            both.insert(both.end(), back->begin(), back->end());
+            return std::make_shared<const std::vector<std::complex<double>>>(std::move(both));
+        });
+    }
+
     // Stage twiddles of a smooth_catalog.h kernel.
     int smooth_table(const SmoothEntry& e) {
         std::vector<int> key(e.radices, e.radices + e.nstages);
         key.push_back(-2);  // distinct from the other table layouts of the radices
         auto it = seq_tables.find(key);
         if (it != seq_tables.end()) return it->second;
-        const int id = add_table(smooth_twiddles(e));
+        const int id = stage_row_table(std::vector<int>(e.radices, e.radices + e.nstages), false);
         seq_tables[key] = id;
         return id;
     }
@@ -535,24 +652,7 @@ struct Builder {
 
     // The Bluestein (rader false) or Rader entries of this precision: conv_catalog.h, or bluestein_catalog.h
     // (whose entries serve both) for plans that may run on the fused multi-pass kernels.
-    std::vector<BlueEntry> conv_choices(bool rader) {
-        std::vector<BlueEntry> out;
-        int count = 0;
-        const BlueEntry* old = blue_entries(&count);
-        if (req.fused_passes) {
-            for (int i = 0; i < count; ++i)
-                if (old[i].dbl == (req.dbl ? 1 : 0)) out.push_back(old[i]);
-            return out;
-        }
-        for (int i = 0; const ConvEntry* c = conv_entry(i); ++i) {
-            if (c->dbl != (req.dbl ? 1 : 0) || (c->rader != 0) != rader) continue;
-            if (static_cast<int64_t>(c->w) * c->pitch * cs > smem_limit) continue;
-            BlueEntry e{count + c->id, c->dbl, c->kind, c->n, c->tpl, c->w, c->maxt, {}, c->nstages};
-            std::copy(c->radices, c->radices + c->nstages, e.radices);
-            out.push_back(e);
-        }
-        return out;
-    }
+    const ConvChoices& conv_choices(bool rader) const { return conv_choice_table(req.dbl, rader, req.fused_passes); }
 
     // Kernel and twiddles of a pass on entry `e` of conv_choices.
     void use_conv(PassSpec& ps, const BlueEntry& e) {
@@ -567,25 +667,35 @@ struct Builder {
         const bool pair = c.kind == kBlueFused || c.kind == kBlueRowsConv;
         key.push_back(pair ? -3 : -2);  // -2: the table of smooth_table
         auto it = seq_tables.find(key);
-        if (it == seq_tables.end()) it = seq_tables.emplace(key, add_table(conv_twiddles(c))).first;
+        if (it == seq_tables.end())
+            it = seq_tables.emplace(key, stage_row_table(std::vector<int>(c.radices, c.radices + c.nstages), pair)).first;
         ps.tables.smooth = it->second;
     }
 
-    // What a convolution of `points` points takes on these entries: their timed cost per point, or (entries
-    // of bluestein_catalog.h) the points alone.
-    double conv_time(int64_t points, std::initializer_list<const BlueEntry*> es) {
-        int count = 0;
-        blue_entries(&count);
-        double c = 0;
-        for (const BlueEntry* e : es) c += e->id < count ? 1.0 : conv_entry(e->id - count)->cost;
-        return c * static_cast<double>(points);
-    }
-
-    // The inverse column kernel of a length.
-    static const BlueEntry* inverse_of(const std::vector<BlueEntry>& cat, const BlueEntry& fwd) {
-        for (const BlueEntry& e : cat)
-            if (e.kind == kBlueColsInv && e.n == fwd.n) return &e;
-        return nullptr;
+    // The column and row kernels of a convolution of `least` to `most` points (M = n1 * n2) whose three passes take
+    // the least time; of equals the pair nearest a square. None: the pointers stay null.
+    void split_convolution(const ConvChoices& cat, int64_t least, int64_t most, const BlueEntry*& cf, const BlueEntry*& rc,
+                           const BlueEntry*& ci) {
+        double best = 0;
+        const int ps_shift = pad_shift_for(req.dbl);
+        for (const ConvChoice& a : cat.kind[kBlueColsFwd]) {
+            if (a.smem > smem_limit || int64_t(a.e.n) * a.e.w * cs > smem_limit) continue;
+            if (!a.inverse || a.inverse->smem > smem_limit) continue;
+            for (const ConvChoice& b : cat.kind[kBlueRowsConv]) {
+                const int64_t M = int64_t(a.e.n) * b.e.n;
+                if (M < least || M > most || b.smem > smem_limit) continue;
+                const double t = (a.cost + b.cost + a.inverse->cost) * static_cast<double>(M);
+                if (cf && t > best) continue;
+                if (int64_t(kmode_pitch(b.e.n, ps_shift)) * cs > smem_limit) continue;
+                if (!cf || t < best ||
+                    std::abs(std::log(double(b.e.n) / a.e.n)) < std::abs(std::log(double(rc->n) / cf->n))) {
+                    best = t;
+                    cf = &a.e;
+                    rc = &b.e;
+                    ci = &a.inverse->e;
+                }
+            }
+        }
     }
 
     // Rader on the size-specialised Bluestein kernels (contiguous axes, prime L): with g a
@@ -599,42 +709,21 @@ struct Builder {
     bool rader_fixed(int ax, int64_t L, int64_t O, Buf& cur) {
         if (req.no_fixed || req.no_rader || L < 3 || L > (int64_t(1) << 30) || !is_prime(L)) return false;
         const int64_t M = L - 1;
-        const std::vector<BlueEntry> cat = conv_choices(true);
-        const int count = static_cast<int>(cat.size());
+        const ConvChoices& cat = conv_choices(true);
         const int ps_shift = pad_shift_for(req.dbl);
+        auto row_fits = [&](const ConvChoice& c) {
+            return c.smem <= smem_limit && int64_t(kmode_pitch(c.e.n, ps_shift)) * cs <= smem_limit;
+        };
         const BlueEntry* fused = nullptr;
-        for (int i = 0; i < count && !fused; ++i) {
-            const BlueEntry& e = cat[i];
-            if (e.dbl == (req.dbl ? 1 : 0) && e.kind == kBlueFused && e.n == M &&
-                int64_t(kmode_pitch(e.n, ps_shift)) * cs <= smem_limit)
-                fused = &e;
-        }
+        for (const ConvChoice& c : cat.kind[kBlueFused])
+            if (!fused && c.e.n == M && row_fits(c)) fused = &c.e;
         // three passes only where Bluestein would take three too (its one block reads and writes HBM once)
         bool one_block = false;
         if (!fused && !req.fused_passes)
-            for (const BlueEntry& e : conv_choices(false))
-                one_block = one_block || (e.kind == kBlueFused && e.n >= 2 * L - 2 &&
-                                          int64_t(kmode_pitch(e.n, ps_shift)) * cs <= smem_limit);
+            for (const ConvChoice& c : conv_choices(false).kind[kBlueFused])
+                one_block = one_block || (c.e.n >= 2 * L - 2 && row_fits(c));
         const BlueEntry *cf = nullptr, *rc = nullptr, *ci = nullptr;
-        double least = 0;
-        for (int i = 0; i < count && !fused && !one_block; ++i) {
-            const BlueEntry& a = cat[i];
-            if (a.kind != kBlueColsFwd || M % a.n || int64_t(a.n) * a.w * cs > smem_limit) continue;
-            const BlueEntry* inv = inverse_of(cat, a);
-            for (int k = 0; k < count && inv; ++k) {
-                const BlueEntry& b = cat[k];
-                if (b.kind != kBlueRowsConv || int64_t(a.n) * b.n != M) continue;
-                if (int64_t(kmode_pitch(b.n, ps_shift)) * cs > smem_limit) continue;
-                const double t = conv_time(M, {&a, &b, inv});
-                if (!cf || t < least ||
-                    (t == least && std::abs(std::log(double(b.n) / a.n)) < std::abs(std::log(double(rc->n) / cf->n)))) {
-                    least = t;
-                    cf = &a;
-                    rc = &b;
-                    ci = inv;
-                }
-            }
-        }
+        if (!fused && !one_block) split_convolution(cat, M, M, cf, rc, ci);
         if (!fused && !(cf && rc && ci)) return false;
 
         const int sgn = req.direction;
@@ -812,47 +901,27 @@ struct Builder {
     // kernel (n2) in three passes. Returns false (generic kernels) when the catalog has no such length.
     bool bluestein_fixed(int ax, int64_t L, int64_t O, Buf& cur) {
         if (req.no_fixed) return false;
-        const std::vector<BlueEntry> cat = conv_choices(false);
-        const int count = static_cast<int>(cat.size());
+        const ConvChoices& cat = conv_choices(false);
         const int64_t need = 2 * L - 2;
         const int ps_shift = pad_shift_for(req.dbl);
         const BlueEntry* fused = nullptr;
-        for (int i = 0; i < count; ++i) {
-            const BlueEntry& e = cat[i];
-            if (e.dbl != (req.dbl ? 1 : 0) || e.kind != kBlueFused || e.n < need) continue;
-            if (int64_t(kmode_pitch(e.n, ps_shift)) * cs > smem_limit) continue;
-            if (!fused || conv_time(e.n, {&e}) < conv_time(fused->n, {fused})) fused = &e;
+        double fused_time = 0;
+        for (const ConvChoice& c : cat.kind[kBlueFused]) {
+            if (c.e.n < need || c.smem > smem_limit || int64_t(kmode_pitch(c.e.n, ps_shift)) * cs > smem_limit) continue;
+            const double t = c.cost * static_cast<double>(c.e.n);
+            if (fused && t >= fused_time) continue;
+            fused = &c.e;
+            fused_time = t;
         }
         const BlueEntry *cf = nullptr, *rc = nullptr, *ci = nullptr;
-        int64_t best = 0;
-        double least = 0;
-        for (int i = 0; i < count && !fused; ++i) {
-            const BlueEntry& a = cat[i];
-            if (a.kind != kBlueColsFwd || int64_t(a.n) * a.w * cs > smem_limit) continue;
-            const BlueEntry* inv = inverse_of(cat, a);
-            for (int k = 0; k < count && inv; ++k) {
-                const BlueEntry& b = cat[k];
-                if (b.kind != kBlueRowsConv) continue;
-                const int64_t M = int64_t(a.n) * b.n;
-                if (M < need || int64_t(kmode_pitch(b.n, ps_shift)) * cs > smem_limit) continue;
-                const double t = conv_time(M, {&a, &b, inv});
-                if (!cf || t < least ||
-                    (t == least && std::abs(std::log(double(b.n) / a.n)) < std::abs(std::log(double(rc->n) / cf->n)))) {
-                    least = t;
-                    best = M;
-                    cf = &a;
-                    rc = &b;
-                    ci = inv;
-                }
-            }
-        }
+        if (!fused) split_convolution(cat, need, kNoLimit, cf, rc, ci);
         if (!fused && !(cf && rc && ci)) return false;
 
         const bool bwd = req.direction == 1;
         (void)bwd;
         const int sgn = req.direction;
         const int64_t E = static_cast<int64_t>(plan.elements);
-        const int64_t M = fused ? fused->n : best;
+        const int64_t M = fused ? fused->n : int64_t(cf->n) * rc->n;
         std::vector<std::complex<double>> chirp, kern;
         if (!req.device_spectrum) chirp_tables(L, M, sgn, chirp, kern);
         const int chirp_id = req.device_spectrum ? add_device_table(L) : add_table(std::move(chirp));
@@ -1736,22 +1805,6 @@ const SmoothEntry* smooth_piped_entry(int id) {
 }
 
 namespace {
-// Per stage the rows W_(ns*R)^(r*jm), jm < ns, r = smooth_tw_power(R, row).
-std::vector<std::complex<double>> stage_rows(const std::vector<int>& radices) {
-    std::vector<int64_t> key(radices.begin(), radices.end());
-    key.push_back(-600);
-    return *cached_table(key, [&] {
-        std::vector<std::complex<double>> t;
-        int64_t ns = 1;
-        for (int R : radices) {
-            for (int q = 0; q < smooth_tw_entries(R); ++q)
-                for (int64_t jm = 0; jm < ns; ++jm) t.push_back(cis_neg(smooth_tw_power(R, q) * jm, ns * R));
-            ns *= R;
-        }
-        return t;
-    });
-}
-
 const std::vector<ConvEntry>& all_conv_entries() {
     static const std::vector<ConvEntry> all = {
 #define SFB_X(ID, DBL, KIND, RADER, N, TPL, W, PADS, PITCH, MAXT, MINB, COST, ...) \
@@ -1764,23 +1817,12 @@ const std::vector<ConvEntry>& all_conv_entries() {
 }  // namespace
 
 std::vector<std::complex<double>> smooth_twiddles(const SmoothEntry& e) {
-    return stage_rows(std::vector<int>(e.radices, e.radices + e.nstages));
+    return *stage_rows(std::vector<int>(e.radices, e.radices + e.nstages));
 }
 
 const ConvEntry* conv_entry(int id) {
     const auto& all = all_conv_entries();
     return id >= 0 && id < static_cast<int>(all.size()) ? &all[id] : nullptr;
-}
-
-std::vector<std::complex<double>> conv_twiddles(const ConvEntry& e) {
-    std::vector<int> r(e.radices, e.radices + e.nstages);
-    auto t = stage_rows(r);
-    if (e.kind == kBlueFused || e.kind == kBlueRowsConv) {
-        std::reverse(r.begin(), r.end());
-        const auto back = stage_rows(r);
-        t.insert(t.end(), back.begin(), back.end());
-    }
-    return t;
 }
 
 int strided_line_kind(const LineLayout& in, const LineLayout& out) {
@@ -1879,7 +1921,7 @@ PlanSpec make_plan(const PlanRequest& req) {
         if (!((req.skip_axes >> ax) & 1u)) plan.transform_size *= req.shape[ax];
     plan.scale = normalization_scale(req.normalization, req.direction, plan.transform_size);
     if (plan.elements > (uint64_t(1) << 40)) throw std::invalid_argument("FFT too large for one device");
-    Builder b{plan, req, req.dbl ? 16 : 8, req.smem_limit > 0 ? req.smem_limit : kSmemDefault, {}};
+    Builder b{plan, req, req.dbl ? 16 : 8, req.smem_limit > 0 ? req.smem_limit : kSmemDefault, {}, {}};
     Buf cur = Buf::Input;
     const int rank = static_cast<int>(req.shape.size());
     const int64_t E = static_cast<int64_t>(plan.elements);
@@ -1903,6 +1945,7 @@ PlanSpec make_plan(const PlanRequest& req) {
         const std::vector<int> r = lean_radix15(ps);
         if (!r.empty()) ps.p.fft1 = b.make_seq(static_cast<int>(ps.p.n), r, ps.kc.maxv, &ps.tables.tw1);
     }
+    b.finish_tables();
     // The batch is the outermost index of every pass: the pass's outer count when it has
     // one (n_outer > 1 or strided columns), else its line count.
     for (auto& ps : plan.passes) {

@@ -167,8 +167,6 @@ const ConvEntry* conv_entry(int id);
 inline int64_t conv_index_bytes(const ConvEntry& e) {
     return e.rader && e.kind == kBlueColsInv ? int64_t(e.n) * e.w * 4 : 0;
 }
-// Its stage twiddles: the rows of smooth_twiddles over its radices, then (convolutions) over the reverse.
-std::vector<std::complex<double>> conv_twiddles(const ConvEntry& e);
 
 // One entry of tc_catalog.h (split-precision tensor-core kernels, complex<float> only).
 struct TcEntry {
@@ -178,6 +176,8 @@ struct TcEntry {
 };
 // Entry for a line length and layout (cols: the lines are adjacent columns), or nullptr.
 const TcEntry* find_tc(int n, bool cols);
+
+enum class TableChoice { all, read, none };
 
 struct PlanRequest {
     bool dbl = false;
@@ -220,6 +220,9 @@ struct PlanRequest {
     bool fused_passes = false;
     // prime lengths L take Bluestein's convolution even where the catalog covers L - 1 (Rader)
     bool no_rader = false;
+    // Which tables make_plan generates: every one (emulation), those that a kernel of the plan reads, or none (a
+    // description of the plan).
+    TableChoice tables = TableChoice::all;
 };
 
 // A Bluestein axis whose chirp and chirp spectrum the provider generates on the device
@@ -242,6 +245,9 @@ struct PlanSpec {
     // Entries of each table; a table whose data is empty but whose size is not is generated on
     // the device (Bluestein chirp and spectrum with PlanRequest::device_spectrum).
     std::vector<size_t> table_sizes;
+    // Whether a kernel of the plan reads the table. A pass on a smooth_catalog.h or conv_catalog.h kernel reads
+    // that kernel's stage table instead of tw1, tw2 (unless the fused multi-pass kernels, an opt-in, take it).
+    std::vector<char> table_read;
     std::vector<std::vector<int32_t>> index_tables;  // int32 tables (Rader permutations)
     std::vector<PassSpec> passes;
     uint64_t scratch_elements = 0;

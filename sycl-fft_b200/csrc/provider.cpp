@@ -421,7 +421,7 @@ void pack_table(const std::vector<std::complex<double>>& t, unsigned char* blob,
 }
 
 DevicePlan* create_plan(const syclfft_b200_plan_config_v1& cfg, uint32_t flags = 0, uint32_t skip_axes = 0,
-                        const LineLayout* line_in = nullptr, const LineLayout* line_out = nullptr);
+                        const LineLayout* line_in = nullptr, const LineLayout* line_out = nullptr, bool spec_only = false);
 void execute_plan(DevicePlan* plan, const void* in, void* out, cudaStream_t stream, uint64_t batch = 0,
                   int direction = 0, int normalization = -1);
 
@@ -446,11 +446,11 @@ DevicePlan* spectrum_plan(int device, int64_t M) {
     return p;
 }
 
-DevicePlan* build_plan(PlanRequest req, int device, uint32_t flags, const std::string& tuning);
+DevicePlan* build_plan(PlanRequest req, int device, uint32_t flags, const std::string& tuning, bool spec_only = false);
 PlanRequest tune(const PlanRequest& req, int device, std::string* report);
 
 DevicePlan* create_plan(const syclfft_b200_plan_config_v1& cfg, uint32_t flags, uint32_t skip_axes,
-                        const LineLayout* line_in, const LineLayout* line_out) {
+                        const LineLayout* line_in, const LineLayout* line_out, bool spec_only) {
     if (cfg.abi_version != SYCLFFT_B200_PROVIDER_ABI_VERSION) throw std::runtime_error("B200 provider ABI mismatch");
     if (cfg.scalar != SYCLFFT_B200_SCALAR_FLOAT && cfg.scalar != SYCLFFT_B200_SCALAR_DOUBLE)
         throw std::invalid_argument("unsupported scalar type");
@@ -483,7 +483,7 @@ DevicePlan* create_plan(const syclfft_b200_plan_config_v1& cfg, uint32_t flags, 
     if (const char* k = std::getenv("SYCLFFT_B200_FUSED4_SINGLE")) req.fused_single = std::strcmp(k, "1") == 0;
     if (const char* k = std::getenv("SYCLFFT_B200_FUSED4")) {
         if (std::strcmp(k, "1") != 0) req.fused_single = false;
-        req.fused_passes = std::strcmp(k, "1") == 0;
+        req.fused_passes = k[0] == '1';
     } else {
         req.fused_single = false;  // the fused kernels are opt-in
     }
@@ -506,39 +506,45 @@ DevicePlan* create_plan(const syclfft_b200_plan_config_v1& cfg, uint32_t flags, 
     std::string tuning;
     if (cfg.measure) {
         // planning_mode::measure: time the candidate decompositions and kernels
-        (void)make_plan(req);  // argument validation before any device work
+        PlanRequest checked = req;  // argument validation before any device work
+        checked.device_spectrum = true;
+        checked.tables = TableChoice::none;
+        (void)make_plan(checked);
         req = tune(req, device, &tuning);
     }
-    return build_plan(req, device, flags, tuning);
+    return build_plan(req, device, flags, tuning, spec_only);
 }
 
-DevicePlan* build_plan(PlanRequest req, int device, uint32_t flags, const std::string& tuning) {
+// spec_only: the description, the status word and the wait limit of a plan that is never executed (the complex
+// plan of a one-pass real transform).
+DevicePlan* build_plan(PlanRequest req, int device, uint32_t flags, const std::string& tuning, bool spec_only) {
     int smem_optin = 0;
     check(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device), "cudaDeviceGetAttribute");
     req.smem_limit = smem_optin;
     req.device_spectrum = true;
+    req.tables = spec_only ? TableChoice::none : TableChoice::read;
     if (flags & SYCLFFT_B200_CREATE_SPLIT_BF16) req.split_bf16 = !req.dbl;
 
     auto plan = std::make_unique<DevicePlan>();
     plan->device = device;
     plan->spec = make_plan(req);
     plan->spec.tuning = tuning;
+    plan->status = status_pool().acquire();
+    plan->owns_status = true;
+    // failure-detection testing: SYCLFFT_B200_WAIT_POLLS sets the wait limit of new plans
+    if (const char* v = std::getenv("SYCLFFT_B200_WAIT_POLLS")) {
+        char* end = nullptr;
+        const long long polls = std::strtoll(v, &end, 10);
+        if (end != v && polls >= 0) plan->wait_polls = polls;
+    }
+    check(cudaDeviceGetAttribute(&plan->sms, cudaDevAttrMultiProcessorCount, device), "cudaDeviceGetAttribute");
+    if (spec_only) return plan.release();
     const size_t cs = req.dbl ? 16 : 8;
 
     // All tables in one allocation, each 256-byte aligned: the complex tables (cast to the
     // plan precision), then the int32 index tables.
-    // A pass on a smooth_catalog.h or conv_catalog.h kernel reads that kernel's stage table instead of tw1, tw2 (unless the fused
-    // multi-pass kernels, an opt-in, take it): tables no kernel reads are not uploaded.
-    const char* f4env = std::getenv("SYCLFFT_B200_FUSED4");
-    const bool fused_opt_in = f4env && f4env[0] == '1';
-    std::vector<char> read(plan->spec.tables.size(), fused_opt_in ? 1 : 0);
-    for (const PassSpec& ps : plan->spec.passes) {
-        const TableIds& t = ps.tables;
-        const bool own = ps.smooth_id >= 0 || ps.conv_id >= 0;
-        for (int id : {own ? -1 : t.tw1, own ? -1 : t.tw2, t.premul, t.pointwise, t.postmul, t.tw4_hi, t.tw4_lo, t.tc_tw,
-                       t.cl_base, t.smooth, t.spiped})
-            if (id >= 0) read[id] = 1;
-    }
+    // Tables no kernel reads are neither made nor uploaded.
+    const std::vector<char>& read = plan->spec.table_read;
     std::vector<size_t> offsets(plan->spec.tables.size()), ioffsets(plan->spec.index_tables.size());
     size_t total = 0;
     for (size_t i = 0; i < plan->spec.tables.size(); ++i) {
@@ -568,15 +574,6 @@ DevicePlan* build_plan(PlanRequest req, int device, uint32_t flags, const std::s
     staging.release(blob, ms);
     check(up, "plan table upload");
     plan->table_bytes = table_bytes;
-    plan->status = status_pool().acquire();
-    plan->owns_status = true;
-    // failure-detection testing: SYCLFFT_B200_WAIT_POLLS sets the wait limit of new plans
-    if (const char* v = std::getenv("SYCLFFT_B200_WAIT_POLLS")) {
-        char* end = nullptr;
-        const long long polls = std::strtoll(v, &end, 10);
-        if (end != v && polls >= 0) plan->wait_polls = polls;
-    }
-    check(cudaDeviceGetAttribute(&plan->sms, cudaDevAttrMultiProcessorCount, device), "cudaDeviceGetAttribute");
     plan->stream_scratch = (flags & SYCLFFT_B200_CREATE_STREAM_SCRATCH) != 0;
     if (plan->spec.scratch_elements && !plan->stream_scratch) {
         check(cudaMallocAsync(&plan->scratch, plan->spec.scratch_elements * cs, ms), "cudaMallocAsync(scratch)");
@@ -656,8 +653,7 @@ DevicePlan* build_plan(PlanRequest req, int device, uint32_t flags, const std::s
     // four-step column + row passes (and Bluestein's three passes) of a contiguous axis with a
     // fused kernel: one launch, the intermediate in an L2-resident ring. Opt-in
     // (SYCLFFT_B200_FUSED4=1): measured slower than the separate launches on B200.
-    const char* f4 = std::getenv("SYCLFFT_B200_FUSED4");
-    const bool fused_ok = f4 && f4[0] == '1' && !req.no_fixed;
+    const bool fused_ok = req.fused_passes && !req.no_fixed;
     for (size_t i = 0; fused_ok && i + 1 < plan->passes.size(); ++i) {
         const PassSpec& a = plan->passes[i].spec_ref();
         const PassSpec& b = plan->passes[i + 1].spec_ref();
@@ -783,7 +779,8 @@ DevicePlan* create_real_plan_1d(const syclfft_b200_plan_config_v1& cfg, int kind
     ic.in_place = 0;
     ic.normalization = 0;
     if (smooth) ic.measure = 0;
-    std::unique_ptr<DevicePlan> inner(create_plan(ic, flags | SYCLFFT_B200_CREATE_SYNC));
+    // the one-pass form executes nothing of its complex plan
+    std::unique_ptr<DevicePlan> inner(create_plan(ic, flags | SYCLFFT_B200_CREATE_SYNC, 0, nullptr, nullptr, smooth != nullptr));
     if (smooth) inner->spec.tuning = report;
     auto plan = std::make_unique<DevicePlan>();
     plan->device = inner->device;
@@ -1889,7 +1886,8 @@ PlanRequest tune(const PlanRequest& req, int device, std::string* report) {
         std::string desc;
         try {
             PlanRequest rd = r;
-            rd.device_spectrum = true;  // the description does not need the chirp spectra
+            rd.device_spectrum = true;
+            rd.tables = TableChoice::none;
             desc = describe_plan(make_plan(rd));
         } catch (...) {
             continue;

@@ -158,3 +158,15 @@ def narrow_lines(kind, feat, w, n_cols, n_outer):
     o, c = np.zeros(n_cols * n_outer, np.int64), np.zeros(n_cols * n_outer, np.int64)
     n = L.narrow_lines(kind, feat, w, n_cols, n_outer, o.ctypes.data, c.ctypes.data)
     return None if n < 0 else (o[:n], c[:n])
+
+
+def tables_left_out(shape, batch, double=False, fused=False):
+    """Tables of the plan that no kernel reads and that are therefore not made; asserts that the others are."""
+    L = _load("libtables_check.so")
+    L.tables_left_out.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.c_uint, ctypes.c_void_p, ctypes.c_uint64, ctypes.c_char_p,
+                                  ctypes.c_size_t]
+    sh = (ctypes.c_uint64 * 3)(*(list(shape) + [0] * (3 - len(shape))))
+    why = ctypes.create_string_buffer(256)
+    n = L.tables_left_out(int(double), int(fused), len(shape), sh, batch, why, 256)
+    assert n >= 0, (shape, batch, double, why.value.decode())
+    return n

@@ -254,3 +254,18 @@ def test_lean_radix15_stages():
             if p["lean"]:
                 pos = [order.index(r) for r in p["radices"]]
                 assert pos == sorted(pos), (n, p["radices"])
+
+
+def test_only_tables_that_a_kernel_reads_are_made():
+    """A plan makes the stage tables of the kernels that run its passes and none of those they replace; with the
+    fused multi-pass kernels in play every table is made."""
+    from native_libs import tables_left_out
+
+    for double in (False, True):
+        for shape, batch in SHAPES:
+            tables_left_out(shape, batch, double)
+            assert tables_left_out(shape, batch, double, fused=True) == 0
+        assert tables_left_out([3000], 4, double) >= 1       # of the runtime-length kernel
+        assert tables_left_out([680400], 2, double) >= 2     # of both four-step passes
+        assert tables_left_out([4099], 2, double) >= 1
+        assert tables_left_out([1 << 24], 1, double) == 0    # fixed or runtime-length kernels run it
