@@ -515,6 +515,10 @@ DevicePlan* create_plan(const syclfft_b200_plan_config_v1& cfg, uint32_t flags, 
     return build_plan(req, device, flags, tuning, spec_only);
 }
 
+// Loads the size-specialised kernel that runs a pass on the current device (kernel_set.hpp): a plan's first execute
+// finds it loaded.
+void load_kernels(const BoundPass& bp, int sms);
+
 // spec_only: the description, the status word and the wait limit of a plan that is never executed (the complex
 // plan of a one-pass real transform).
 DevicePlan* build_plan(PlanRequest req, int device, uint32_t flags, const std::string& tuning, bool spec_only) {
@@ -649,6 +653,7 @@ DevicePlan* build_plan(PlanRequest req, int device, uint32_t flags, const std::s
         bp.spiped_tw = tab(ps.tables.spiped);
         bp.conv = conv_entry(ps.conv_id);
         plan->passes.push_back(bp);
+        load_kernels(bp, plan->sms);
     }
     // four-step column + row passes (and Bluestein's three passes) of a contiguous axis with a
     // fused kernel: one launch, the intermediate in an L2-resident ring. Opt-in
@@ -831,6 +836,11 @@ DevicePlan* create_real_plan_1d(const syclfft_b200_plan_config_v1& cfg, int kind
             table.insert(table.end(), u.begin(), u.end());
         }
     }
+    if (smooth)
+        check(plan->real_spiped && static_cast<int64_t>(cfg.batch_count) > plan->sms
+                  ? prepare_smooth_piped(*plan->real_spiped)
+                  : prepare_smooth(*smooth, static_cast<int64_t>(cfg.batch_count), 1),
+              "real transform kernel");
     std::vector<unsigned char> tw(table.size() * cs);
     for (size_t k = 0; k < table.size(); ++k) {
         if (dbl) {
@@ -1374,6 +1384,17 @@ SmoothParams to_smooth(const PassParams& p, const void* tw, int64_t* n_outer) {
     s.tw4_shift = p.tw4_shift;
     s.tw4_conj = p.tw4_sign > 0 ? 1 : 0;
     return s;
+}
+
+void load_kernels(const BoundPass& bp, int sms) {
+    if (bp.smooth) {
+        int64_t n_outer = 1;
+        const SmoothParams s = to_smooth(bp.p, nullptr, &n_outer);
+        check(bp.spiped && s.n_cols > sms ? prepare_smooth_piped(*bp.spiped) : prepare_smooth(*bp.smooth, s.n_cols, n_outer),
+              "FFT kernel");
+    } else if (bp.conv) {
+        check(prepare_conv(*bp.conv), "FFT convolution kernel");
+    }
 }
 
 // Launches one bound pass of a plan on its kernel family.

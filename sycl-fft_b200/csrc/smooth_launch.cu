@@ -14,14 +14,19 @@ static_assert(SFB_SMOOTH_PARTS == 24, "SFB_EACH_PART lists the parts");
 #define SFB_EACH_CONV_PART(F) F(0) F(1) F(2) F(3) F(4) F(5) F(6) F(7)
 static_assert(SFB_CONV_PARTS == 8, "SFB_EACH_CONV_PART lists the parts");
 
-#define SFB_DECL(P) const SmoothKernel* smooth_part_##P(int* count); const SmoothKernel* smooth_run_part_##P(int* count);
+// a part of smooth_catalog.h is compiled in three objects and one of its run-on forms, one of conv_catalog.h in two
+#define SFB_DECL(P)                                       \
+    const SmoothKernel* smooth_part_##P##_0(int* count);  \
+    const SmoothKernel* smooth_part_##P##_1(int* count);  \
+    const SmoothKernel* smooth_part_##P##_2(int* count);  \
+    const SmoothKernel* smooth_run_part_##P(int* count);
 SFB_EACH_PART(SFB_DECL)
 #undef SFB_DECL
 #define SFB_EACH_SPIPED_PART(F) F(0) F(1) F(2) F(3)
 #define SFB_DECL(P) const SmoothKernel* smooth_piped_part_##P(int* count);
 SFB_EACH_SPIPED_PART(SFB_DECL)
 #undef SFB_DECL
-#define SFB_DECL(P) const ConvKernel* conv_part_##P(int* count);
+#define SFB_DECL(P) const ConvKernel* conv_part_##P##_0(int* count); const ConvKernel* conv_part_##P##_1(int* count);
 SFB_EACH_CONV_PART(SFB_DECL)
 #undef SFB_DECL
 
@@ -30,7 +35,7 @@ namespace {
 KernelSet& smooth_kernels() {
     static KernelSet* k = [] {
         auto* s = new KernelSet;
-#define SFB_ADD(P) s->add(smooth_part_##P);
+#define SFB_ADD(P) s->add(smooth_part_##P##_0); s->add(smooth_part_##P##_1); s->add(smooth_part_##P##_2);
         SFB_EACH_PART(SFB_ADD)
 #undef SFB_ADD
         s->finish();
@@ -66,7 +71,7 @@ KernelSet& smooth_piped_kernels() {
 KernelSet& conv_kernels() {
     static KernelSet* k = [] {
         auto* s = new KernelSet;
-#define SFB_ADD(P) s->add(conv_part_##P);
+#define SFB_ADD(P) s->add(conv_part_##P##_0); s->add(conv_part_##P##_1);
         SFB_EACH_CONV_PART(SFB_ADD)
 #undef SFB_ADD
         s->finish();
@@ -75,7 +80,22 @@ KernelSet& conv_kernels() {
     return *k;
 }
 
+// The most dynamic shared memory a launch of the entry takes.
+size_t smooth_smem(const SmoothEntry& e) { return static_cast<size_t>(e.w) * e.pitch * (e.dbl ? 16 : 8); }
+size_t conv_smem(const ConvEntry& e) { return static_cast<size_t>(e.w) * e.pitch * (e.dbl ? 16 : 8) + conv_index_bytes(e); }
+
 }  // namespace
+
+cudaError_t prepare_smooth(const SmoothEntry& e, int64_t n_cols, int64_t n_outer) {
+    return (smooth_runs_on(e.kind, e.feat, e.w, n_cols, n_outer) ? smooth_run_kernels() : smooth_kernels())
+        .prepare(e.id, smooth_smem(e));
+}
+
+cudaError_t prepare_smooth_piped(const SmoothEntry& e) {
+    return smooth_piped_kernels().prepare(e.id, static_cast<size_t>(smooth_piped_smem(e.n, e.pitch)));
+}
+
+cudaError_t prepare_conv(const ConvEntry& e) { return conv_kernels().prepare(e.id, conv_smem(e)); }
 
 cudaError_t launch_smooth(const SmoothEntry& e, SmoothParams p, int64_t n_outer, int sms, const void* in, void* out,
                           cudaStream_t stream) {
@@ -95,7 +115,7 @@ cudaError_t launch_smooth(const SmoothEntry& e, SmoothParams p, int64_t n_outer,
     p.col_tiles = (p.n_cols + p.w - 1) / p.w;
     void* args[] = {&p, const_cast<void**>(&in), &out};
     return (run ? smooth_run_kernels() : smooth_kernels())
-        .launch(e.id, n_outer * p.col_tiles, threads, p.w * line, e.w * line, args, stream);
+        .launch(e.id, n_outer * p.col_tiles, threads, p.w * line, smooth_smem(e), args, stream);
 }
 
 cudaError_t launch_smooth_piped(const SmoothEntry& e, const SmoothParams& p, int sms, int* status, long long wait_polls,
@@ -123,7 +143,7 @@ cudaError_t launch_conv(const ConvEntry& e, FixedParams p, int64_t n_outer, int 
     p.col_tiles = (p.n_cols + p.w - 1) / p.w;
     const size_t extra = conv_index_bytes(e);
     void* args[] = {&p, const_cast<void**>(&in), &out};
-    return conv_kernels().launch(e.id, n_outer * p.col_tiles, threads, p.w * line + extra, e.w * line + extra, args, stream);
+    return conv_kernels().launch(e.id, n_outer * p.col_tiles, threads, p.w * line + extra, conv_smem(e), args, stream);
 }
 
 }  // namespace sfb

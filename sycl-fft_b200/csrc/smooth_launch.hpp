@@ -21,7 +21,11 @@ cudaError_t launch_smooth(const SmoothEntry& e, SmoothParams p, int64_t n_outer,
 cudaError_t launch_smooth_piped(const SmoothEntry& e, const SmoothParams& p, int sms, int* status, long long wait_polls,
                                 const void* in, void* out, cudaStream_t stream);
 
-// One kernel of a compiled part of the catalog.
+// Loads the kernel that a pass of this size takes (the pipelined form), so that its first launch need not.
+cudaError_t prepare_smooth(const SmoothEntry& e, int64_t n_cols, int64_t n_outer);
+cudaError_t prepare_smooth_piped(const SmoothEntry& e);
+
+// One kernel of a compiled part of the catalog (nullptr: in another object of the part).
 struct SmoothKernel {
     int id;
     const void* fn;

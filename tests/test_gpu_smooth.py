@@ -185,3 +185,29 @@ def test_narrow_arrays(sf, torch, shape, batch, dbl):
             got = big.cpu().numpy()
             assert rel_l2(got[:n * (batch - 1)], ref[:n * (batch - 1)]) <= tol(n, dbl)
             assert np.all(got[n * (batch - 1):] == 9.0)
+
+
+@pytest.mark.parametrize("n,batch,dbl,kind", [(1458, 5, False, "c2c"), (1372, 3, True, "c2c"), (9408, 150, False, "c2c"), (2861, 3, False, "c2c"),
+                                              (26 * 525, 2, False, "r2c"), (9000, 2, True, "c2c")], ids=str)
+def test_first_execute_under_capture(sf, torch, n, batch, dbl, kind):
+    """A plan loads its kernels when it is made, so that its very first execute can be captured."""
+    s = "double" if dbl else "float"
+    if kind == "r2c":
+        x = np.random.default_rng(n).uniform(-1, 1, (batch, n)).astype(np.float32)
+        p = sf.plan_dft_r2c_1d(s, n, batch)
+        ref = np.fft.rfft(x.astype(np.float64), axis=1)
+    else:
+        x = uniform_complex(n * batch, n, np.complex128 if dbl else np.complex64)
+        p = sf.plan_many_dft(s, [n], batch, sf.direction.forward)
+        ref = fp64_fft(x, [n], batch, -1)
+    a = torch.from_numpy(x).cuda()
+    o = torch.zeros(ref.shape, dtype=torch.complex128 if dbl else torch.complex64, device="cuda")
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        p.execute(a, o)
+    assert torch.count_nonzero(o) == 0
+    g.replay()
+    torch.cuda.synchronize()
+    assert rel_l2(o.cpu().numpy(), ref) <= tol(n, dbl)
+    del g
