@@ -1957,6 +1957,22 @@ PlanSpec make_plan(const PlanRequest& req) {
     return plan;
 }
 
+// The kernel family that runs a pass, in the order in which the launch looks for one. "smooth" takes its pipelined
+// form where the entry has one and there are more lines than SMs; "piped", "cluster_pipe" and "tma" need 16-byte
+// aligned buffers and otherwise leave the pass to the next family it is planned for.
+static const char* pass_kernel(const PassSpec& ps) {
+    if (ps.smooth_id >= 0) return "smooth";
+    if (ps.conv_id >= 0) return "conv";
+    if (ps.blue_id >= 0) return "bluestein";
+    if (ps.tc_id >= 0) return "tensor_core";
+    if (ps.piped_id >= 0) return "piped";
+    if (ps.cluster_pipe) return "cluster_pipe";
+    if (ps.cluster_id >= 0) return "cluster";
+    if (ps.tma) return "tma";
+    if (ps.fixed_id >= 0) return "fixed";
+    return ps.lean ? "lean" : "general";
+}
+
 std::string describe_plan(const PlanSpec& plan) {
     std::ostringstream os;
     os << "{\"elements\":" << plan.elements << ",\"scratch_elements\":" << plan.scratch_elements
@@ -1973,6 +1989,7 @@ std::string describe_plan(const PlanSpec& plan) {
            << ",\"threads\":" << ps.threads << ",\"smem\":" << ps.smem_bytes << ",\"tiles\":" << p.tiles
            << ",\"maxv\":" << ps.kc.maxv << ",\"maxt\":" << ps.kc.maxt << ",\"src\":" << int(ps.src)
            << ",\"dst\":" << int(ps.dst) << ",\"bytes\":" << ps.bytes_moved
+           << ",\"kernel\":\"" << pass_kernel(ps) << "\""
            << ",\"store_via_smem\":" << p.store_via_smem << ",\"fixed_id\":" << ps.fixed_id
            << ",\"piped_id\":" << ps.piped_id << ",\"spiped_id\":" << ps.spiped_id << ",\"tc_id\":" << ps.tc_id << ",\"blue_id\":" << ps.blue_id << ",\"tma\":" << (ps.tma ? 1 : 0) << ",\"cluster_id\":" << ps.cluster_id << ",\"cluster_pipe\":" << (ps.cluster_pipe ? 1 : 0) << ",\"cluster\":[" << ps.cl_n1 << "," << ps.cl_n2 << ","
            << ps.cl_p << "],\"rader\":" << (ps.rader ? 1 : 0) << ",\"lean\":" << (ps.lean ? 1 : 0)

@@ -205,3 +205,15 @@ def test_narrow_arrays_fill_their_tiles(w):
             assert np.array_equal(got[0] * cols + got[1], np.arange(cols * outer)) and got[1].max() == cols - 1
         for kind, feat in ((CC, 1), (KK, 0), (CK, 0), (KC, 0)):
             assert narrow_lines(kind, feat, w, cols, 3) is None
+
+
+def test_described_kernels():
+    """`kernel` names the family that runs a pass, whatever other families it is planned for besides."""
+    def names(shape, **kw):
+        return [p["kernel"] for p in describe(shape, 4, **kw)["passes"]]
+
+    assert names([3000]) == ["smooth"] and names([4096]) == ["smooth"] and names([680400]) == ["smooth", "smooth"]
+    assert names([13440]) == ["piped"] and names([64]) == ["fixed"] and names([64], double=True) == ["smooth"]
+    assert names([15]) == ["lean"] and names([1 << 24]) == ["lean", "lean"] and names([7]) == ["general"]
+    assert names([1009]) == ["conv"] and names([65537]) == ["conv"] * 3 and names([1009, 6])[1] == "general"
+    assert names([256], split_bf16=True) == ["tensor_core"]
