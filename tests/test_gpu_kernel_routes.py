@@ -1,5 +1,7 @@
-"""Kernels that other lengths or batches than the everyday ones reach: the runtime-length kernel of contiguous lines.
-FP64 references at the complex tolerance of the length."""
+"""Kernels that other lengths or batches than the everyday ones reach: the runtime-length kernel of contiguous lines,
+the pipelined 7-smooth lines (their plain form for a few lines, and the copy wait that gives up). FP64 references at the complex tolerance of the length."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -43,3 +45,47 @@ def test_runtime_length_kernel(sf, torch, n, batch, dbl, kernels):
         o = torch.full_like(a, 9.0)
         p.execute(a, o).synchronize()
         assert rel_l2(o.cpu().numpy(), fp64_fft(x, [n], batch, d, norm_scale(norm, d, n))) <= tol(n, dbl)
+
+
+@pytest.mark.parametrize("few", [1, 100, 148])
+def test_pipelined_plan_runs_a_few_lines(sf, torch, few):
+    n, batch = 12544, 297
+    p = sf.plan_many_dft("float", [n], batch, sf.direction.forward)
+    assert p.describe()["passes"][0]["spiped_id"] >= 0
+    x = uniform_complex(n * few, few, np.complex64)
+    a = torch.from_numpy(x).cuda()
+    o = torch.full((n * batch,), 9.0, dtype=a.dtype, device="cuda")
+    err = ctypes.create_string_buffer(1024)
+    rc = p._lib.syclfft_b200_execute_batch(p._handle, a.data_ptr(), o.data_ptr(), few,
+                                           torch.cuda.current_stream().cuda_stream, err, 1024)
+    assert rc == 0, err.value
+    got = o.cpu().numpy()
+    assert rel_l2(got[:n * few], fp64_fft(x, [n], few, -1)) <= tol(n) and np.all(got[n * few:] == 9.0)
+
+
+@pytest.mark.parametrize("kind", ["c2c", "r2c"])
+def test_pipelined_line_wait_that_gives_up(sf, torch, kind):
+    """With a wait limit of 0 polls every block gives up its first copy wait, lets the copy land and returns: the
+    event raises execution_failed once, and the default limit then computes the transform."""
+    if kind == "c2c":
+        n, batch = 12544, 297
+        x = uniform_complex(n * batch, n, np.complex64)
+        p = sf.plan_many_dft("float", [n], batch, sf.direction.forward)
+        ref, out = fp64_fft(x, [n], batch, -1), (batch * n,)
+    else:
+        n, batch = 26880, 150
+        x = np.random.default_rng(n).uniform(-1, 1, (batch, n)).astype(np.float32)
+        p = sf.plan_dft_r2c_1d("float", n, batch)
+        ref, out = np.fft.rfft(x.astype(np.float64), axis=1), (batch, n // 2 + 1)
+    a = torch.from_numpy(x).cuda()
+    o = torch.zeros(out, dtype=torch.complex64, device="cuda")
+    assert p._lib.syclfft_b200_plan_set_wait_limit(p._handle, 0) == 0
+    ev = p.execute(a, o)
+    with pytest.raises(sf.SyclfftError) as info:
+        ev.synchronize()
+    assert info.value.code == sf.error_code.execution_failed
+    assert p._lib.syclfft_b200_plan_status(p._handle) == 0  # reported once, then cleared
+    ev.synchronize()
+    assert p._lib.syclfft_b200_plan_set_wait_limit(p._handle, -1) == 0
+    p.execute(a, o).synchronize()
+    assert rel_l2(o.cpu().numpy(), ref) <= tol(n)
