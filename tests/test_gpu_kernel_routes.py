@@ -1,5 +1,6 @@
 """Kernels that other lengths or batches than the everyday ones reach: the runtime-length kernel of contiguous lines,
-the pipelined 7-smooth lines (their plain form for a few lines, and the copy wait that gives up). FP64 references at the complex tolerance of the length."""
+the pipelined 7-smooth lines (their plain form for a few lines, and the copy wait that gives up), and the one-pass
+real kernels of SYCLFFT_B200_REAL_FUSED=fixed. FP64 references at the complex tolerance of the length."""
 import ctypes
 
 import numpy as np
@@ -89,3 +90,20 @@ def test_pipelined_line_wait_that_gives_up(sf, torch, kind):
     assert p._lib.syclfft_b200_plan_set_wait_limit(p._handle, -1) == 0
     p.execute(a, o).synchronize()
     assert rel_l2(o.cpu().numpy(), ref) <= tol(n)
+
+
+@pytest.mark.parametrize("n,dbl", [(512, False), (2048, False), (8192, False), (512, True), (4096, True)])
+def test_fixed_real_kernels(sf, torch, n, dbl, monkeypatch):
+    """The power-of-two one-pass real kernels that SYCLFFT_B200_REAL_FUSED=fixed asks for."""
+    monkeypatch.setenv("SYCLFFT_B200_REAL_FUSED", "fixed")
+    s, batch = "double" if dbl else "float", 37
+    opts = sf.plan_options(normalization=sf.normalization.orthogonal)
+    f, b = sf.plan_dft_r2c_1d(s, n, batch, opts), sf.plan_dft_c2r_1d(s, n, batch, opts)
+    assert f.launches() == 1 and b.launches() == 1 and f.describe()["fused"] == 1
+    x = np.random.default_rng(n).uniform(-1, 1, (batch, n)).astype(np.float64 if dbl else np.float32)
+    spec = torch.zeros((batch, n // 2 + 1), dtype=f.dtype, device="cuda")
+    back = torch.zeros((batch, n), dtype=b.real_dtype, device="cuda")
+    f.execute(torch.from_numpy(x).cuda(), spec).synchronize()
+    assert rel_l2(spec.cpu().numpy(), np.fft.rfft(x.astype(np.float64), axis=1, norm="ortho")) <= tol(n, dbl)
+    b.execute(spec, back).synchronize()
+    assert rel_l2(back.cpu().numpy(), x.astype(np.float64)) <= 2 * tol(n, dbl)
