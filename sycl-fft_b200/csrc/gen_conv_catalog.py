@@ -1,19 +1,20 @@
 #!/usr/bin/env python
 """Writes conv_catalog.h: the instantiations of conv_kernel.cuh (Bluestein and Rader passes).
 
+    python gen_conv_catalog.py > out               # the committed catalog again (its lines are the timed choices)
     python gen_conv_catalog.py --candidates > candidates.txt   # up to KEEP layouts of every entry
-    python gen_conv_catalog.py chosen.txt > conv_catalog.h     # the catalog of the chosen lines
+    python gen_conv_catalog.py chosen.txt > out    # the catalog of the chosen lines, with their times
 
 Lengths: single-block convolutions of 2^a * {1, 3, 5, 7} points in float; in double and for the two
 factors of a longer convolution those 7-smooth lengths that no longer length beats in time (complex lines
 timed on B200), so a convolution of at least 2L - 2 points pads little and costs no slow length. Layouts come
-from the model of gen_smooth_catalog.py; the committed catalog holds the fastest of them with its time.
+from the model of gen_smooth_catalog.py; the catalog holds the fastest of them with its time at 96 MB.
 Rader passes are made where a prime can need them: a single block of length n when n + 1 is prime, columns
 of a power of two.
 """
 import sys
 
-from gen_smooth_catalog import CC, KK, best
+from gen_smooth_catalog import CC, KK, best, committed, write_catalog, write_parts
 
 KEEP = 9
 FLOAT_FUSED = sorted(f << a for f in (1, 3, 5, 7) for a in range(15) if 64 <= f << a <= 16384)
@@ -69,17 +70,9 @@ HEAD = """// Written by gen_conv_catalog.py: the Bluestein and Rader pass kernel
 
 def write(rows, out):
     out.write(HEAD)
-    parts = 8
-    ident = 0
-    for p in range(parts):
-        out.write("#define SFB_CONV_PART_%d(X) \\\n" % p)
-        text = []
-        for e in rows[p::parts]:
-            text.append("    X(%d, %s)" % (ident, e))
-            ident += 1
-        out.write(" \\\n".join(text) + "\n\n")
-    out.write("#define SFB_CONV_PARTS %d\n" % parts)
-    out.write("#define SFB_CONV_CATALOG(X) %s\n" % " ".join("SFB_CONV_PART_%d(X)" % p for p in range(parts)))
+    write_parts(rows, out, "SFB_CONV", 8)
+    out.write("#define SFB_CONV_PARTS 8\n")
+    write_catalog(out, "SFB_CONV", 8)
 
 
 def main():
@@ -91,7 +84,7 @@ def main():
         with open(arg) as f:
             write([line.strip() for line in f if line.strip()], sys.stdout)
     else:
-        write([rows[0] for rows in candidates()], sys.stdout)
+        write(committed("conv_catalog.h"), sys.stdout)
 
 
 if __name__ == "__main__":

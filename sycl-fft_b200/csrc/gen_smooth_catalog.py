@@ -1,9 +1,11 @@
 #!/usr/bin/env python
 """Writes smooth_catalog.h: the instantiations of smooth_kernel.cuh, one per 7-smooth length, precision
-and thread mapping.
+and thread mapping; and smooth_piped_catalog.h, their copy-engine-pipelined forms.
 
+    python gen_smooth_catalog.py > out            # the committed catalog again (its lines are the timed choices)
     python gen_smooth_catalog.py --candidates > candidates.txt   # up to KEEP layouts of every entry
-    python gen_smooth_catalog.py chosen.txt > smooth_catalog.h   # the catalog of the chosen lines
+    python gen_smooth_catalog.py chosen.txt > out # the catalog of the chosen lines
+    python gen_smooth_catalog.py --piped [--candidates | chosen.txt]   # the same of smooth_piped_catalog.h
 
 For every length the generator enumerates the radix sequences of the fewest stages (and one more),
 the threads per line, and the shared-memory row layouts, and ranks them under a model of one SM's
@@ -15,9 +17,16 @@ complex length is left out where the power-of-two kernel of fixed_catalog.h was 
 lines). The real transforms (FEAT 2 and 4) take the layouts chosen for complex lines, or one with a radix
 above 16 where that was faster for them. Radices above 16 (float only; the values
 of a double butterfly would take twice the registers) are taken where they timed at least 1.5% below the best layout of radices to 16.
+A time is the best of three runs of three launches on 128 MB (column mappings: 1024 columns), every candidate in one
+process; the chosen lines are the catalogs themselves, which the generator reads back.
+
+Pipelined candidates: the even float lines above 4096 points, one per block, on the layouts timed for the plain
+kernel whose copy buffer fits beside them; those that timed at least 5% below the plain kernel are in the catalog.
 """
 import itertools
 import math
+import os
+import re
 import sys
 
 KK, CC, CK, KC = 0, 1, 2, 3
@@ -298,33 +307,81 @@ HEAD = """// Written by gen_smooth_catalog.py: the size-specialised kernels of t
 """
 
 
-def write(rows, out):
-    out.write(HEAD)
-    parts = 24
+PIPED_HEAD = """// Written by gen_smooth_catalog.py --piped: the copy-engine-pipelined 7-smooth kernels (smooth_piped.cuh): even float
+// lines of 4116 to 14400 points, those that timed at least 5% below the plain kernel of smooth_catalog.h (128 MB of
+// lines).
+//
+// X(ID, DOUBLE, KIND, FEAT, N, TPL, W, PADS, PITCH, MAXT, MINB, RADICES...) as in smooth_catalog.h; KIND 0, W 1;
+// FEAT 2: R2C of twice the length; MINB blocks fit an SM beside their copy buffers.
+// SFB_SPIPED_PART_<p> lists the entries that smooth_piped_variants.cu compiles as part p.
+#pragma once
+
+"""
+
+
+def write_parts(rows, out, macro, parts):
+    """Row i goes to part i mod parts; ids number the entries in the order of the parts."""
     ident = 0
     for p in range(parts):
-        out.write("#define SFB_SMOOTH_PART_%d(X) \\\n" % p)
+        out.write("#define %s_PART_%d(X) \\\n" % (macro, p))
         text = []
         for e in rows[p::parts]:
             text.append("    X(%d, %s)" % (ident, e))
             ident += 1
         out.write(" \\\n".join(text) + "\n\n")
-    out.write("#define SFB_SMOOTH_PARTS %d\n" % parts)
-    out.write("#define SFB_SMOOTH_CATALOG(X) %s\n" % " ".join("SFB_SMOOTH_PART_%d(X)" % p for p in range(parts)))
+
+
+def write_catalog(out, macro, parts):
+    out.write("#define %s_CATALOG(X) %s\n" % (macro, " ".join("%s_PART_%d(X)" % (macro, p) for p in range(parts))))
+
+
+def write(rows, out):
+    out.write(HEAD)
+    write_parts(rows, out, "SFB_SMOOTH", 24)
+    out.write("#define SFB_SMOOTH_PARTS 24\n")
+    write_catalog(out, "SFB_SMOOTH", 24)
+
+
+def write_piped(rows, out):
+    out.write(PIPED_HEAD)
+    write_parts(rows, out, "SFB_SPIPED", 4)
+    write_catalog(out, "SFB_SPIPED", 4)
+
+
+def committed(name):
+    """The rows of a committed catalog, in the order in which write_parts was given them."""
+    with open(os.path.join(os.path.dirname(os.path.abspath(__file__)), name)) as f:
+        parts = [re.findall(r"X\(\d+, ([-0-9, ]+)\)", part) for part in f.read().split("#define ")[1:] if "_PART_" in part.split("(")[0]]
+    return [part[i] for i in range(max(map(len, parts))) for part in parts if i < len(part)]
+
+
+def piped_candidates():
+    """Pipelined forms of the plain float layouts, complex lines and R2C."""
+    for n in range(4097, 16385):
+        if n % 2 or not smooth(n):
+            continue
+        for feat in (0, 2):
+            for l in best(0, KK, n):
+                room = SMEM // ((n + l.pitch) * 8 + 16 + 1024)
+                if l.w == 1 and room >= 1:
+                    e = entry(l, feat).split(", ")
+                    e[9] = str(min(int(e[9]), room))
+                    yield ", ".join(e)
 
 
 def main():
-    # --candidates: one timed candidate per line; a file of chosen lines (the fastest of each length,
-    # type and mapping): the catalog of those; no argument: the model's first choice everywhere
-    arg = sys.argv[1] if len(sys.argv) > 1 else ""
+    args = sys.argv[1:]
+    piped = args[:1] == ["--piped"]
+    arg = args[piped] if len(args) > piped else ""
+    put = write_piped if piped else write
     if arg == "--candidates":
-        for rows in candidates().values():
+        for rows in [piped_candidates()] if piped else candidates().values():
             print("\n".join(rows))
     elif arg:
         with open(arg) as f:
-            write([line.strip() for line in f if line.strip()], sys.stdout)
+            put([line.strip() for line in f if line.strip()], sys.stdout)
     else:
-        write([rows[0] for rows in candidates().values()], sys.stdout)
+        put(committed("smooth_piped_catalog.h" if piped else "smooth_catalog.h"), sys.stdout)
 
 
 if __name__ == "__main__":

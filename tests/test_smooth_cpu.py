@@ -217,3 +217,14 @@ def test_described_kernels():
     assert names([15]) == ["lean"] and names([1 << 24]) == ["lean", "lean"] and names([7]) == ["general"]
     assert names([1009]) == ["conv"] and names([65537]) == ["conv"] * 3 and names([1009, 6])[1] == "general"
     assert names([256], split_bf16=True) == ["tensor_core"]
+
+
+@pytest.mark.parametrize("args,name", [(["gen_smooth_catalog.py"], "smooth_catalog.h"),
+                                       (["gen_smooth_catalog.py", "--piped"], "smooth_piped_catalog.h"),
+                                       (["gen_conv_catalog.py"], "conv_catalog.h")], ids=lambda v: str(v[-1]))
+def test_generators_write_the_committed_catalogs(args, name):
+    import subprocess
+    import sys
+    csrc = os.path.join(os.path.dirname(__file__), "..", "sycl-fft_b200", "csrc")
+    out = subprocess.run([sys.executable, "-B"] + args, cwd=csrc, capture_output=True, text=True, check=True).stdout
+    assert out == open(os.path.join(csrc, name)).read()
