@@ -868,9 +868,7 @@ def run_serve_devtime(args):
         lib.syclfft_b200_describe_plan(h, desc, len(desc))
         passes = json.loads(desc.value.decode())["passes"]
         shape[(n, dbl)] = ("c128 " if dbl else "c64 ") + "+".join(
-            q["kind"] + ("(lean)" if q.get("lean") else
-                         "(general)" if max(q["fixed_id"], q["blue_id"], q["piped_id"], q["cluster_id"], q["tc_id"]) < 0
-                         else "") for q in passes)
+            q["kind"] + (f"({q['kernel']})" if q["kernel"] in ("lean", "general") else "") for q in passes)
     most = {False: 0, True: 0}
     for r in reqs:
         most[r.double] = max(most[r.double], r.elements)

@@ -12,11 +12,12 @@
 // points: 77 -> 66 us; double, 8.4 M points: 80 -> 64 us).
 //
 // What bounds it: exchanges and issue slots (convolution kernels run at 100 to 270 G points/s in float, HBM
-// would allow about 400), the Rader gather and scatter the 32-byte sectors their 8- or 16-byte accesses
-// take (65537 points x 256, float: 106 and 103 us of 285). Convolution lengths are chosen by the passes'
-// timed cost per point (conv_catalog.h): the smallest length is often slower than one a little longer
-// (double 28927: 210 x 288 = 60480 points 227 us, 64 x 960 = 61440 points 192 us). Against the kernels of
-// bluestein_catalog.h, 110 primes from 11 to 65537: 1.25x float, 1.15x double (geometric mean).
+// would allow about 400; the 65537-point rows: issue 77%, load/store data pipe 71%), the Rader gather and scatter the
+// 32-byte sectors their 8- or 16-byte accesses take (65537 points x 256, float: 109 and 103 us of 285 to 298).
+// Convolution lengths are chosen by the passes' timed cost per point (conv_catalog.h): the smallest length is often
+// slower than one a little longer (double 28927: 210 x 288 = 60480 points 227 us, 64 x 960 = 61440 points 192 us).
+// Against the kernels of bluestein_catalog.h, 106 primes from 11 to 65537 at 32 MB: 1.24x float, 1.13x double
+// (geometric means; none slower).
 #pragma once
 
 #include <cuda_runtime.h>

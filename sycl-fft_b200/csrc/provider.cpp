@@ -804,7 +804,7 @@ DevicePlan* create_real_plan_1d(const syclfft_b200_plan_config_v1& cfg, int kind
     const uint64_t h = n / 2;
     // One pass when N/2 has a smooth_catalog.h kernel with the pre- / post-process (not for split-precision
     // plans, whose inner FFT runs on the tensor cores): 1.03x to 1.4x the power-of-two kernels of real_kernel.cu
-    // and 2.1x (geometric mean over 286 lengths) the two-pass form. SYCLFFT_B200_REAL_FUSED=0 keeps the two-pass
+    // and 2.4x (geometric mean over 681 lengths) the forms before it. SYCLFFT_B200_REAL_FUSED=0 keeps the two-pass
     // form, =fixed the kernels of real_kernel.cu.
     const char* fused_env = std::getenv("SYCLFFT_B200_REAL_FUSED");
     const bool split = !dbl && (flags & SYCLFFT_B200_CREATE_SPLIT_BF16) != 0;
@@ -1154,7 +1154,7 @@ DevicePlan* create_strided_plan(const syclfft_b200_plan_config_v1& cfg, const sy
     if (cfg.rank == 1) {
         // Lines whose sides are each contiguous lines or adjacent columns: where the length has a
         // smooth_catalog.h kernel of those mappings it reads and writes the layouts itself, one HBM pass
-        // instead of two or three (1024 points x 65536, float, columns -> rows: 397 -> 224 us;
+        // instead of two or three (1024 points x 65536, float, columns -> rows: 391 to 403 -> 206 to 224 us;
         // 177 lengths of 64 MB matrices 2.4 to 2.7x). planning_mode::measure times both forms.
         const LineLayout li = line_of(in), lo = line_of(out);
         const bool dbl = cfg.scalar == SYCLFFT_B200_SCALAR_DOUBLE;
@@ -1404,7 +1404,7 @@ void launch_bound_pass(DevicePlan* plan, const BoundPass& bp, void* src, void* d
     if (bp.smooth) {
         int64_t n_outer = 1;
         SmoothParams sp = to_smooth(bp.p, bp.smooth_tw, &n_outer);
-        if (bp.spiped && aligned && sp.n_cols > plan->sms) {
+        if (bp.spiped && aligned && sp.n_cols > plan->sms) {  // the line is measured in smooth_piped.cuh
             sp.tw = bp.spiped_tw;
             check(launch_smooth_piped(*bp.spiped, sp, plan->sms, plan->status, bp.spiped_polls, src, dst, stream),
                   "FFT pipelined pass launch");

@@ -13,7 +13,7 @@
 // These two are for the lengths without a one-pass kernel (half lengths with a factor above 7, or longer
 // than a block holds); 7-smooth half lengths run on smooth_kernel.cuh with the process fused into the
 // transform. The power-of-two kernels below (kFeatRealPre / kFeatRealPost of fixed_kernel.cuh) do the
-// same; they are taken under SYCLFFT_B200_REAL_FUSED=fixed.
+// same; they are taken under SYCLFFT_B200_REAL_FUSED=fixed and SYCLFFT_B200_KERNELS=generic.
 #include <atomic>
 #include <type_traits>
 

@@ -9,23 +9,25 @@
 //  * radices 6, 9, 10, 12, 14 and 15 next to the powers of two and 3, 5, 7, so that lengths with odd
 //    factors take three or four stages instead of five to seven; an odd radix first where there is one:
 //    its exchange then falls in distinct banks without padding, which saves the padding's address
-//    arithmetic in every stage (3000 points: [8, 15, 5, 5] padded 197 us, [15, 8, 5, 5] without 156 us).
+//    arithmetic in every stage (3000 points x 16384, bare launches on one card: [8, 15, 5, 5] padded 196 us,
+//    [15, 8, 5, 5] without 166 us).
 //  * float radices to 32 at up to 128 registers a thread: 256 to 1024 points in two stages, longer lines in
-//    three. Shared-memory traffic (the load/store pipe was 66 to 78% busy) and barriers fall with every
-//    exchange, and the values in flight per SM rise. [15, 8, 5, 5] -> [25, 10, 12]: 3000 x 16384 178 -> 151
-//    to 161 us (several cards); 810 x 840 four-step [9, 9, 10] and [15, 4, 14] -> [27, 30] and [30, 28]: 680400 x 64 360 -> 310 to 326 us;
-//    1024 columns -> rows [16, 8, 8] -> [32, 32]: 240 -> 209 to 224 us. 869 of the 1820 float entries, those that
-//    gained at least 1.5%: 1.15x (geometric mean). Packed two-value additions (add.f32x2) in their place
-//    gave nothing: the exchanges, not the arithmetic, fill the time.
+//    three. Shared-memory traffic and barriers fall with every exchange, and the values in flight per SM rise.
+//    [15, 8, 5, 5] -> [25, 10, 12] in the same launches: 166 -> 160 us; 810 x 840 four-step [9, 9, 10] and
+//    [15, 4, 14] -> [27, 30] and [30, 28]: 680400 x 64 360 -> 310 to 326 us; 1024 columns -> rows [16, 8, 8] ->
+//    [32, 32]: 240 -> 209 to 224 us (ranges: several cards). 869 of the 1820 float entries, those that gained at
+//    least 1.5%: 1.15x (geometric mean). Packed two-value additions (add.f32x2) in their place gave nothing: the
+//    exchanges, not the arithmetic, fill the time.
 //  * up to 16 values a thread in double too, at 128 registers and half the threads: the same bytes in
 //    flight with one exchange less (2048 points: [8, 8, 8, 4] 180 us, [16, 16, 8] 168 us per 1.07 GB).
 //
-// What bounds it: HBM for the lines up to about 2000 points (4.9 to 6.4 of the 6.5 TB/s copy rate), the
-// issue slots and exchanges of the longer ones, one or two blocks of which fill an SM. Times per execute on
-// B200 against the runtime-length kernels: 3000 x 16384 float 337 -> 161 us, 680400 x 64 float (810 x 840
-// four-step) 638 -> 326 us, 840 x 1200 x 4 float 101 -> 34 us; complex<double> 65536 x 512 (256 x 256)
-// 415 -> 354 us against fixed_kernel.cuh. All 691 whole-line lengths above 15: 1.96x (geometric mean, 64 MB
-// batches), columns 2.3x, four-steps to 2^20 1.67x.
+// What bounds it: HBM for the lines up to about 2000 points (4.9 to 6.4 of the 6.5 TB/s copy rate), the issue slots
+// and exchanges of the longer ones (3000 points: issue 67%, load/store data pipe 64%, DRAM 56%; 4096: 63, 61 and
+// 64%), one or two blocks of the longest of which fill an SM. Times per execute on B200 against the runtime-length
+// kernels: 3000 x 16384 float 338 -> 155 to 161 us, 680400 x 64 float (810 x 840 four-step) 640 -> 316 to 326 us,
+// 840 x 1200 x 4 float 101 -> 34 us; complex<double> 65536 x 512 (256 x 256) 402 to 421 -> 341 to 357 us against
+// fixed_kernel.cuh. The catalog's 680 whole-line lengths: 2.06x (geometric mean, 64 MB), columns of 64-column arrays
+// 1.9x (354 lengths), four-steps to 2^20 1.78x (619 lengths), real lines 2.4x (681); none of them slower.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -55,10 +57,9 @@ struct SmoothParams {
 };
 
 // Twiddles of one butterfly, u[r] *= w^r with w = W_(Ns*R)^jm. The table holds w, w^2, w^4 and w^8 for every
-// jm (rows of Ns entries, so lanes read them coalesced) and the other powers take at most two products:
-// against the powers of w alone (error 1.7e-7 -> 1.2e-7 at 3000 points, that of a full table) for the time
-// of neither more than 4% above them nor below a full table's R - 1 loads (3000 points x 16384: 155 us
-// powers, 166 us this, 172 us full table at 4 blocks per SM; 4096: 172, 174, 182).
+// jm (rows of Ns entries, so lanes read them coalesced) and the other powers take at most two products: the error of a
+// full table (3000 points: 1.2e-7, 1.7e-7 from the powers of w alone) for 1% (4096 points, three stages of 16) to 7%
+// (3000 points as [15, 8, 5, 5]) more time than the powers alone, where a full table's R - 1 loads took another 4%.
 template <int R, int NS, class C>
 __device__ __forceinline__ void smooth_twiddle(C* u, const C* __restrict__ tw, int jm) {
     const C w1 = __ldg(tw + jm);
@@ -198,7 +199,6 @@ __device__ __forceinline__ void smooth_stage(SmoothCtx<T>& X) {
         const int j = t + i * TPL;
         if (act && (EXACT || i + 1 < NB || j < NR)) {
             if constexpr (FIRST && !(FEAT & kSmoothPre)) {
-
                 if (X.in_ok) {
                     const C* g = CMAP ? X.gin + (int64_t)j * X.in_ks : X.gin + j;
 #pragma unroll

@@ -11,8 +11,12 @@
 //
 // Taken by the even lengths that timed at least 5% below the plain kernel (56 of 228; 128 MB of lines: 1.16x
 // complex, 1.15x R2C; 12544 points 80 -> 66 us), where there are more lines than SMs: the first line of a CTA
-// hides behind nothing. R2C 26880 x 4096: 307 -> 253 us, now bound by the exchanges of one CTA per SM (three
-// stages and the pairs' pass). Shorter lines mostly lose: two copy buffers per SM displace blocks.
+// hides behind nothing. Pipelined over plain time, the 56 entries at 38 line counts: from 149 to 444 lines 0.82 to
+// 1.19, 0.99 in the geometric mean (a half-full last round costs either form more or less), from 445 lines 0.91, from
+// 1185 0.90. A higher line would cost the lengths that gain from the first line on (12544 points: 0.87 at 180 lines)
+// what it gives the others (12096: 1.14). R2C 26880 x 4096: 307 -> 249 to 253 us, bound by the exchanges of one CTA
+// per SM (three stages and the pairs' pass: issue 52%, load/store data pipe 54%, DRAM 36%). Shorter lines mostly
+// lose: two copy buffers per SM displace blocks.
 //
 // Waits on the copy are bounded: after Q.wait_polls polls the CTA records a timeout in the
 // plan's status word, lets the copy it gave up on land (bounded again by kSpinLimit, so no
